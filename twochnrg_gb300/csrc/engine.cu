@@ -155,6 +155,9 @@ struct nrg_ctx {
   static constexpr int kMaxSplit = 8;
   cudaStream_t aux[kMaxSplit] = {};
   cudaEvent_t fork = nullptr, join[kMaxSplit] = {};
+  // the row kernel beside the cluster kernel of the middle blocks
+  cudaStream_t rows_stream = nullptr;
+  cudaEvent_t rows_fork = nullptr, rows_join = nullptr;
   nrg::DevBuf gpart_k[kMaxSplit], gbig;
   // mixed precision: per concurrent grid the blocked reduction's [V W], column
   // and share scratch, and the tensor-core product's slices
@@ -275,7 +278,7 @@ void check_flag(nrg_ctx* c) {
   if (f & DEV_DEGEN_OVERFLOW) throw NrgError(NRG_ERR_SIZE, "too many near-degenerate levels for SetDegen");
   if (f & DEV_BAD_INPUT) throw NrgError(NRG_ERR_ARG, "non-finite value met in an eigenvalue solve");
   if (f & DEV_NOT_CONVERGED) throw NrgError(NRG_ERR_NOT_CONVERGED, "inverse iteration did not converge");
-  if (f & DEV_TIMEOUT) throw NrgError(NRG_ERR_TIMEOUT, "a tensor-core kernel's bounded wait gave up");
+  if (f & DEV_TIMEOUT) throw NrgError(NRG_ERR_TIMEOUT, "a kernel's bounded wait gave up");
 }
 
 // ------------------------------------------------------------------ eigensolve
@@ -325,6 +328,26 @@ int cluster_threads(bool shared_gpu) {
   const char* s = std::getenv("NRG_CLUSTER_THREADS");
   if (s) return std::atoi(s) == 256 ? 256 : 512;
   return shared_gpu ? 256 : 512;
+}
+
+// Blocks up to this many states go to the row kernel (k_rows.cu), as long as
+// their rows fit in the shared memory of a cluster of 16 (617 states on a
+// GB300): 1.9 times faster than the lower-triangle cluster kernel at 600 states
+// (6.14 against 11.6 ms), 3.6 times at 256, 5.4 times at 64.
+int rows_block_threshold() {
+  const char* s = std::getenv("NRG_ROWS_N");
+  return s ? std::atoi(s) : 617;
+}
+
+// Its cluster size: 16 CTAs from 33 states on (256 states: 0.914 ms, on 8
+// 1.32, on 4 2.1 ms; the 21 blocks of a one-channel iteration together 0.99,
+// 1.34, 2.15 ms), 8 for smaller blocks, where the CTAs would have one row or
+// none (32 states: 64 us on 8, 67 on 16).  Also for the workers of
+// nrg_sweep_batch (16 sweeps: 1.27 s on 16, 1.35 on 8, 1.33 on 4, 1.40 on 2).
+int choose_rows_cluster(int maxn) {
+  const char* s = std::getenv("NRG_ROWS_CLUSTER");
+  if (s) return std::atoi(s);
+  return maxn > 32 ? 16 : 8;
 }
 
 // Blocks at least this large are tridiagonalized by a cooperative grid of
@@ -586,20 +609,54 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
       c->launches++; c->timing.tridiag_launches++;
     }
   }
-  if (nbig < nb) {
+  // The other blocks: the middle ones by the cluster kernel, those whose rows
+  // fit in a cluster's shared memory by the row kernel beside it.
+  int nrows0 = nbig, rcl = 0, rncl = 0;
+  while (nrows0 < nb && P.bsize[order_h[nrows0]] > rows_block_threshold()) ++nrows0;
+  for (; nrows0 < nb; ++nrows0) {
+    const int maxs = std::max(P.bsize[order_h[nrows0]], 2);
+    rcl = choose_rows_cluster(maxs);
+    rncl = tridiag_rows_max_clusters(rcl, maxs);
+    for (; rncl <= 0 && rcl < 16; ) { rcl *= 2; rncl = tridiag_rows_max_clusters(rcl, maxs); }
+    if (rncl > 0) break;
+  }
+  const bool both = nbig < nrows0 && nrows0 < nb;
+  if (both) {
+    if (!c->rows_stream) {
+      CU(cudaStreamCreateWithFlags(&c->rows_stream, cudaStreamNonBlocking));
+      CU(cudaEventCreateWithFlags(&c->rows_fork, cudaEventDisableTiming));
+      CU(cudaEventCreateWithFlags(&c->rows_join, cudaEventDisableTiming));
+    }
+    CU(cudaEventRecord(c->rows_fork, c->stream));
+  }
+  if (nbig < nrows0) {
     int maxs = P.bsize[order_h[nbig]];
     TridiagArgs ts = ta;
     ts.order = d_order + nbig;
-    ts.nblocks = nb - nbig;
+    ts.nblocks = nrows0 - nbig;
     ts.maxn = std::max(maxs, 2);
     int cluster = choose_cluster(maxs, c->shared_gpu);
     int threads = cluster_threads(c->shared_gpu);
     int ncl = tridiag_max_clusters(cluster, ts.maxn, threads);
     if (ncl <= 0) { cluster = 8; threads = 512; ncl = tridiag_max_clusters(cluster, ts.maxn, threads); }
     if (ncl <= 0) throw NrgError(NRG_ERR_SIZE, "tridiagonalization does not fit on the device");
-    ncl = std::min(ncl, nb - nbig);
+    ncl = std::min(ncl, nrows0 - nbig);
     CU(launch_tridiag(ts, cluster, ncl, c->stream, threads));
     c->launches++; c->timing.tridiag_launches++;
+  }
+  if (nrows0 < nb) {
+    cudaStream_t sr = both ? c->rows_stream : c->stream;
+    if (both) CU(cudaStreamWaitEvent(sr, c->rows_fork, 0));
+    TridiagArgs ts = ta;
+    ts.order = d_order + nrows0;
+    ts.nblocks = nb - nrows0;
+    ts.maxn = std::max(P.bsize[order_h[nrows0]], 2);
+    CU(launch_tridiag_rows(ts, rcl, std::min(rncl, nb - nrows0), sr));
+    c->launches++; c->timing.tridiag_launches++;
+    if (both) {
+      CU(cudaEventRecord(c->rows_join, sr));
+      CU(cudaStreamWaitEvent(c->stream, c->rows_join, 0));
+    }
   }
   for (int k = 0; K > 1 && k < K; ++k) CU(cudaStreamWaitEvent(c->stream, c->join[k], 0));
   if (coop.owns_lock()) {
@@ -3021,6 +3078,9 @@ void nrg_destroy(nrg_ctx* ctx) {
     if (ctx->join[k]) cudaEventDestroy(ctx->join[k]);
   }
   if (ctx->fork) cudaEventDestroy(ctx->fork);
+  if (ctx->rows_stream) { cudaStreamSynchronize(ctx->rows_stream); cudaStreamDestroy(ctx->rows_stream); }
+  if (ctx->rows_fork) cudaEventDestroy(ctx->rows_fork);
+  if (ctx->rows_join) cudaEventDestroy(ctx->rows_join);
   if (ctx->bsync) cudaEventDestroy(ctx->bsync);
   cudaStreamDestroy(ctx->stream);
   delete ctx->tan;

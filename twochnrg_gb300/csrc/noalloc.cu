@@ -18,7 +18,7 @@
 // that makes one warm-up call per device before it carves out its memory, or
 // runs the process with CUDA_MODULE_LOADING=EAGER.
 //
-// The kernels are the ones nrg_diag_blocks runs (k_tridiag.cu, k_tdeig.cu);
+// The kernels are the ones nrg_diag_blocks runs (k_rows.cu, k_tdeig.cu);
 // only the tables they read are generated on the device instead of uploaded.
 #include <cuda_runtime.h>
 
@@ -113,7 +113,9 @@ extern "C" nrg_status nrg_diag_block_noalloc(int n, const double* a, double* eig
   void* p = nullptr;
   if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || !p) return NRG_ERR_CUDA;
   double* base = static_cast<double*>(p);
-  if (tridiag_max_clusters(8, n < 2 ? 2 : n) <= 0) return NRG_ERR_SIZE;
+  int cl = n > 32 ? 16 : 8;  // as nrg_diag_blocks' choice for one block
+  if (tridiag_rows_max_clusters(cl, n < 2 ? 2 : n) <= 0) cl = 8;
+  if (tridiag_rows_max_clusters(cl, n < 2 ? 2 : n) <= 0) return NRG_ERR_SIZE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const Layout L = layout(base);
   const int bw = backtransform_warps(n);
@@ -123,7 +125,7 @@ extern "C" nrg_status nrg_diag_block_noalloc(int n, const double* a, double* eig
   ta.nblocks = 1; ta.order = L.order; ta.bsize = L.bsize; ta.hoff = L.hoff; ta.soff = L.soff;
   ta.H = L.A; ta.d = L.d; ta.e = L.e; ta.tau = L.tau; ta.queue = L.queue; ta.flag = L.flag;
   ta.maxn = n < 2 ? 2 : n;
-  if (launch_tridiag(ta, 8, 1, s) != cudaSuccess) return NRG_ERR_CUDA;
+  if (launch_tridiag_rows(ta, cl, 1, s) != cudaSuccess) return NRG_ERR_CUDA;
   TdEigArgs ea{};
   ea.nblocks = 1; ea.bsize = L.bsize; ea.soff = L.soff; ea.d = L.d; ea.e = L.e; ea.ev = L.ev; ea.nstates = n;
   ea.flag = L.flag; ea.maxn = n; ea.fde = L.fde; ea.e2 = L.e2; ea.split = L.split;
@@ -149,5 +151,6 @@ extern "C" nrg_status nrg_diag_block_noalloc(int n, const double* a, double* eig
   if (flag & DEV_SIZE) return NRG_ERR_SIZE;
   if (flag & DEV_BAD_INPUT) return NRG_ERR_ARG;
   if (flag & DEV_NOT_CONVERGED) return NRG_ERR_NOT_CONVERGED;
+  if (flag & DEV_TIMEOUT) return NRG_ERR_TIMEOUT;
   return NRG_OK;
 }
