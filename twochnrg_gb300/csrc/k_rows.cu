@@ -89,23 +89,6 @@ __device__ __forceinline__ bool try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// 1 / sqrt(x) and 1 / x for normal x: the hardware's approximation (about 22
-// bits) and one step of third order, (1 - e)^(-1/2) = 1 + e/2 + 3 e^2/8 + ...
-// and (1 - e)^-1 = 1 + e + e^2 + ...: five and three FP64 operations in place
-// of the library's ten and six.
-__device__ __forceinline__ double fast_rsqrt(double x) {
-  double r;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-(x * r), r, 1.0);
-  return fma(r * e, fma(0.375, e, 0.5), r);
-}
-__device__ __forceinline__ double fast_rcp(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-x, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
-
 // Sums of RT values over the warp's lanes in RT + log2(32 / RT) additions: the
 // lanes halve the set of values they carry at each of the first steps.  Lane
 // l with l % (32 / RT) == 0 ends with value l / (32 / RT).

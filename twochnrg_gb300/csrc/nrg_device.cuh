@@ -18,6 +18,23 @@ inline int max_dyn_smem() {
 }
 
 #ifdef __CUDACC__
+// 1 / sqrt(x) and 1 / x for normal x: the hardware's approximation (about 22
+// bits) and one step of third order, (1 - e)^(-1/2) = 1 + e/2 + 3 e^2/8 + ...
+// and (1 - e)^-1 = 1 + e + e^2 + ...: five and three FP64 operations in place
+// of the library's ten and six.
+__device__ __forceinline__ double fast_rsqrt(double x) {
+  double r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-(x * r), r, 1.0);
+  return fma(r * e, fma(0.375, e, 0.5), r);
+}
+__device__ __forceinline__ double fast_rcp(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
 // Sum over a full warp in fixed point: every value aligned to the largest
 // exponent with 58 bits, the three 27-bit limbs added by redux.sync, one
 // conversion back.  An FP64 addition holds its sub-partition for 64 cycles and
