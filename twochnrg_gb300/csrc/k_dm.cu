@@ -10,9 +10,11 @@
 // per shell, the partial trace is a gather over per-block term lists, and the
 // frequency dependence is isolated: every shell becomes lists of
 // (E_j - E_i, weight) records once, keeping only the pairs whose term can be
-// nonzero, and the Lehmann kernel stages each chunk of records in shared
-// memory and sums it against a tile of frequencies, with the log-Gaussian /
-// Gaussian kernels of BroadDelta.cpp evaluated on the fly.
+// nonzero.  The lists are summed through moments of bins of their keys
+// (k_fgt.cu); the Lehmann kernel here does the short ones directly, staging each
+// chunk of records in shared memory and summing it against a tile of
+// frequencies, with the log-Gaussian / Gaussian kernels of BroadDelta.cpp
+// evaluated on the fly.
 #include "nrg_device.cuh"
 
 namespace nrg {

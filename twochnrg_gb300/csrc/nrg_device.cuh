@@ -525,6 +525,32 @@ struct LehmannArgs {      // A(omega) = sum_N sum_records w exp(-(t - key)^2) / 
   const int* fold_pos;      // the frequency's position in that list
   double* out;              // [nomega]
 };
+// A list of records summed through moments of bins of its keys (k_fgt.cu).
+constexpr int kFgtMaxBins = 1024;
+constexpr int kFgtTerms = 24;
+constexpr double kFgtBin = 0.125;    // width of a bin in the key
+constexpr double kFgtReach = 27.5;   // exp(-x^2) is 0 beyond
+struct FgtList {
+  const double* key;
+  const double* w;
+  const double* tw;       // tangents [p * tstride + record], as DmRecArgs
+  const double* tg;
+  int64_t tstride;
+  int64_t nrec;
+  double origin;          // key at the first bin's lower edge
+  int nbins, bin0;        // bins; first of the list's in the launch
+  int chunk, nchunks, chunk0;  // records per chunk (a multiple of 256)
+  int* counts;            // [nchunks][nbins]
+  int* start;             // [nbins + 1] records before each bin
+  int* perm;              // [nrec] record indices in bin order
+  double* moments;        // [(1 + 2 ntan) * kFgtTerms][nbins]
+  int shell, gauss, nomega, omega_first;
+  double* part;           // [nomega]
+  double* tpart;          // [p * tpart_stride + j]
+  int64_t tpart_stride;
+};
+void launch_fgt(const LehmannArgs& a, const FgtList* lists, int nlists, const int* chunk_list, int nchunks,
+                const int* bin_list, int nbins, const int* first_warp, int nwarps, int ntan, cudaStream_t s);
 void launch_lehmann(const LehmannArgs& a, cudaStream_t s);       // the items (one shell's lists)
 // The same items over tangent lists: sum (d w + g x) exp(-x^2), x = t - key.
 void launch_lehmann_tangent(const LehmannArgs& a, cudaStream_t s);
