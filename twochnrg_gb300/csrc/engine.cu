@@ -1014,12 +1014,12 @@ void plan_update(UpdatePlan& U, const ModelSpec& m, const Basis& B, const EigPla
             if ((int)U.terms1.size() > first1) {
               const int gid = (int)U.g1first.size();
               U.g1first.push_back(first1); U.g1count.push_back((int)U.terms1.size() - first1);
-              for (int mt = 0; mt * 64 < p.count; ++mt)
-                for (int nt = 0; nt * 64 < J.kj; ++nt) { U.t1group.push_back(gid); U.t1mn.push_back((mt << 16) | nt); }
+              for (int mt = 0; mt * kGemmTile < p.count; ++mt)
+                for (int nt = 0; nt * kGemmTile < J.kj; ++nt) { U.t1group.push_back(gid); U.t1mn.push_back((mt << 16) | nt); }
             }
           }
-        for (int mt = 0; mt * 64 < J.ki; ++mt)
-          for (int nt = 0; nt * 64 < J.kj; ++nt) { U.tjob.push_back(jid); U.tmn.push_back((mt << 16) | nt); }
+        for (int mt = 0; mt * kGemmTile < J.ki; ++mt)
+          for (int nt = 0; nt * kGemmTile < J.kj; ++nt) { U.tjob.push_back(jid); U.tmn.push_back((mt << 16) | nt); }
       }
   }
   U.o_t1 = U.up.add(U.terms1); U.o_g1f = U.up.add(U.g1first); U.o_g1c = U.up.add(U.g1count);
@@ -1070,15 +1070,15 @@ void launch_update_plan(nrg_ctx* c, Timer& tm, UpdatePlan& U, const UpdateInputs
   tm.stop(tu, &c->timing.update_ms);
 }
 
-// Grouped FP64 GEMM jobs (gemm_jobs_kernel): one 64 x 64 tile per CTA.
+// Grouped FP64 GEMM jobs (gemm_jobs_kernel): one tile per CTA.
 struct GemmPlan {
   std::vector<GemmJob> jobs;
   std::vector<int> tjob, tmn;
   void add(const GemmJob& J) {
     const int id = (int)jobs.size();
     jobs.push_back(J);
-    for (int mt = 0; mt * 64 < J.m; ++mt)
-      for (int nt = 0; nt * 64 < J.n; ++nt) { tjob.push_back(id); tmn.push_back((mt << 16) | nt); }
+    for (int mt = 0; mt * kGemmTile < J.m; ++mt)
+      for (int nt = 0; nt * kGemmTile < J.n; ++nt) { tjob.push_back(id); tmn.push_back((mt << 16) | nt); }
   }
 };
 

@@ -15,66 +15,35 @@
 // chunk of records in shared memory and summing it against a tile of
 // frequencies, with the log-Gaussian / Gaussian kernels of BroadDelta.cpp
 // evaluated on the fly.
+#include "gemm_tile.cuh"
 #include "nrg_device.cuh"
 
 namespace nrg {
 
 namespace {
 
-constexpr int TM = 64, TN = 64, TK = 16;
-
-__global__ void __launch_bounds__(256) gemm_jobs_kernel(const GemmJob* jobs, const int* tile_job, const int* tile_mn) {
-  __shared__ double As[TK][TM + 1];
-  __shared__ double Bs[TK][TN];
+__global__ void __launch_bounds__(kGemmThreads, 6) gemm_jobs_kernel(const GemmJob* jobs, const int* tile_job,
+                                                                 const int* tile_mn) {
+  __shared__ GemmSmem S;
   const GemmJob J = jobs[tile_job[blockIdx.x]];
   const int mn = tile_mn[blockIdx.x];
-  const int m0 = (mn >> 16) * TM, n0 = (mn & 0xffff) * TN;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  double acc[4][4];
+  const int m0 = (mn >> 16) * kGemmTile, n0 = (mn & 0xffff) * kGemmTile;
+  const int rows = J.m - m0;
+  double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  auto loadB = [&](int k, int c) { return n0 + c < J.n ? J.B[(int64_t)k * J.ldb + n0 + c] : 0.0; };
+  if (J.transA)
+    gemm_tile<true>(S, J.k, rows, [&](int r, int k) { return r < rows ? J.A[(int64_t)k * J.lda + m0 + r] : 0.0; },
+                    loadB, acc);
+  else
+    gemm_tile<false>(S, J.k, rows, [&](int r, int k) { return r < rows ? J.A[(int64_t)(m0 + r) * J.lda + k] : 0.0; },
+                     loadB, acc);
+  const int c = n0 + (threadIdx.x & 31), r0 = m0 + 8 * (threadIdx.x >> 5);
+  if (c >= J.n) return;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-  for (int k0 = 0; k0 < J.k; k0 += TK) {
-    for (int idx = threadIdx.x; idx < TM * TK; idx += 256) {
-      const int r = idx / TK, c = idx - r * TK;
-      const int gr = m0 + r, gc = k0 + c;
-      double v = 0.0;
-      if (gr < J.m && gc < J.k) v = J.transA ? J.A[(int64_t)gc * J.lda + gr] : J.A[(int64_t)gr * J.lda + gc];
-      As[c][r] = v;
-    }
-    for (int idx = threadIdx.x; idx < TK * TN; idx += 256) {
-      const int r = idx / TN, c = idx - r * TN;
-      const int gr = k0 + r, gc = n0 + c;
-      Bs[r][c] = (gr < J.k && gc < J.n) ? J.B[(int64_t)gr * J.ldb + gc] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < TK; ++kk) {
-      double a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = m0 + ty + 16 * i;
-    if (r >= J.m) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = n0 + tx + 16 * j;
-      if (c < J.n) {
-        double* o = J.C + (int64_t)r * J.ldc + c;
-        *o = J.accum ? *o + acc[i][j] : acc[i][j];
-      }
-    }
+  for (int i = 0; i < 8; ++i) {
+    if (r0 + i >= J.m) break;
+    double* o = J.C + (int64_t)(r0 + i) * J.ldc + c;
+    *o = J.accum ? *o + acc[i] : acc[i];
   }
 }
 
@@ -490,7 +459,7 @@ __global__ void lehmann_fold_kernel(LehmannArgs A) {
 }  // namespace
 
 void launch_gemm_jobs(const GemmJob* jobs, const int* tile_job, const int* tile_mn, int ntiles, cudaStream_t s) {
-  if (ntiles > 0) gemm_jobs_kernel<<<ntiles, 256, 0, s>>>(jobs, tile_job, tile_mn);
+  if (ntiles > 0) gemm_jobs_kernel<<<ntiles, kGemmThreads, 0, s>>>(jobs, tile_job, tile_mn);
 }
 
 void launch_dm_trace(const DmTraceArgs& a, int nblocks, cudaStream_t s) {

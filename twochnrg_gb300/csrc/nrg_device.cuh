@@ -280,6 +280,7 @@ struct ThermoArgs {
 void launch_thermo(const ThermoArgs& a, const int* state_block, int n, double* partial, cudaStream_t s);
 
 // ---------------------------------------------------------------- update
+constexpr int kGemmTile = 32;  // tile of the grouped GEMMs (gemm_tile.cuh)
 struct GatherTerm {       // T[dst rows] += coef * M . Zt[src rows]
   int job;                // rotation job
   int dst_base, dst_stride, rows;   // rows of T (local to the job's T)
@@ -398,7 +399,7 @@ struct GemmJob {          // C (m x n) = op(A) (m x k) . B (k x n), row-major, F
   int ldc;
   int accum;              // 1: C += op(A) . B (after the launches that write C before)
 };
-// One 64x64 tile of C per CTA: tile t belongs to job tile_job[t] at
+// One kGemmTile-square tile of C per CTA: tile t belongs to job tile_job[t] at
 // (tile_mn[t] >> 16, tile_mn[t] & 0xffff).
 void launch_gemm_jobs(const GemmJob* jobs, const int* tile_job, const int* tile_mn, int ntiles, cudaStream_t s);
 
