@@ -28,9 +28,11 @@ namespace nrg {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kBlocks = 304;  // two CTAs per SM for the reductions
+constexpr int kBlocks = 304;  // two CTAs of one warp per SM for the reductions
+constexpr int kMaxAvg = 5;    // averaged operators (two sums each between the 12 thermodynamic and the last)
+constexpr int kEigParts = 4;  // CTAs per block of the division pass
 
-// One CTA per block: dlambda and the coupling matrix C (n x kept, row-major)
+// kEigParts CTAs per block: dlambda and the coupling matrix C (n x kept, row-major)
 // of the block's kept eigenvectors.
 __global__ void __launch_bounds__(kThreads) tan_eig_kernel(TanEigArgs A) {
   const int b = blockIdx.x;
@@ -40,9 +42,10 @@ __global__ void __launch_bounds__(kThreads) tan_eig_kernel(TanEigArgs A) {
   double lmax = 0.0;
   for (int i = 0; i < n; ++i) lmax = fmax(lmax, fabs(lam[i]));
   const double tol = A.degen_tol * fmax(1.0, lmax);
-  for (int x = threadIdx.x; x < n; x += blockDim.x) A.dlam[A.soff[b] + x] = D[(int64_t)x * n + x];
+  const int first = blockIdx.y * blockDim.x + threadIdx.x, stride = gridDim.y * blockDim.x;
+  for (int x = first; x < n; x += stride) A.dlam[A.soff[b] + x] = D[(int64_t)x * n + x];
   double* C = A.C + A.coff[b];
-  for (int idx = threadIdx.x; idx < n * k; idx += blockDim.x) {
+  for (int idx = first; idx < n * k; idx += stride) {
     const int r = idx / k, l = idx - r * k;
     const double gap = lam[l] - lam[r];
     C[idx] = (r == l || fabs(gap) <= tol) ? 0.0 : D[(int64_t)r * n + l] / gap;
@@ -79,9 +82,10 @@ __global__ void tan_scale_kernel(const double* a, double s, int64_t n, double* o
 // per temperature t: sum deg w dE, sum SzSq w dE, sum deg E w dE, with w = e^{-beta_t E};
 // then per averaged operator o over the kept states at betabar:
 // sum deg w dO_ii, sum deg w O_ii dE, and sum deg w dE.
-__global__ void __launch_bounds__(kThreads) tan_sums_kernel(TanSumArgs A, double* partial) {
+__global__ void __launch_bounds__(32) tan_sums_kernel(TanSumArgs A, double* partial) {
   constexpr int W = TanSumArgs::kMaxOut;
   double acc[W];
+#pragma unroll
   for (int t = 0; t < W; ++t) acc[t] = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.nstates; i += gridDim.x * blockDim.x) {
     const int b = A.state_block[i];
@@ -89,6 +93,7 @@ __global__ void __launch_bounds__(kThreads) tan_sums_kernel(TanSumArgs A, double
     const double deg = A.totalS ? 2.0 * S + 1.0 : 1.0;
     const double szsq = A.totalS ? (1.0 / 12.0) * deg * (deg * deg - 1.0) : S * S;
     const double E = A.en[i], dE = A.dE[i];
+#pragma unroll
     for (int t = 0; t < 4; ++t) {
       const double w = exp(-A.beta[t] * E);
       acc[3 * t] += deg * w * dE;
@@ -102,7 +107,9 @@ __global__ void __launch_bounds__(kThreads) tan_sums_kernel(TanSumArgs A, double
     const double deg = A.totalS ? 2.0 * A.kbq[2 * kb + 1] + 1.0 : 1.0;
     const double E = A.ken[i], dE = A.dEk[i];
     const double w = deg * exp(-A.betabar * E);
-    for (int o = 0; o < A.nops; ++o) {
+#pragma unroll
+    for (int o = 0; o < kMaxAvg; ++o) {
+      if (o >= A.nops) break;
       const int64_t off = A.diag_off[o * A.nkblocks + kb];
       const int64_t e = off >= 0 ? off + (int64_t)x * A.kld[kb] + x : -1;
       const double O = e >= 0 ? A.ops[o][e] : 0.0, dO = e >= 0 ? A.dops[o][e] : 0.0;
@@ -111,28 +118,20 @@ __global__ void __launch_bounds__(kThreads) tan_sums_kernel(TanSumArgs A, double
     }
     acc[W - 1] += w * dE;
   }
-  __shared__ double sh[kThreads / 32][W];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
   for (int t = 0; t < W; ++t) {
-    double v = acc[t];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) sh[warp][t] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < W) {
-    double v = 0.0;
-    for (int w = 0; w < kThreads / 32; ++w) v += sh[w][threadIdx.x];
-    partial[(size_t)blockIdx.x * W + threadIdx.x] = v;
+    const double v = warp_sum_fixed(acc[t]);
+    if (threadIdx.x == 0) partial[(size_t)blockIdx.x * W + t] = v;
   }
 }
 
-__global__ void tan_fold_kernel(const double* partial, int nparts, double* out) {
+// One warp per output, lanes over the partials.
+__global__ void __launch_bounds__(32) tan_fold_kernel(const double* partial, int nparts, double* out) {
   constexpr int W = TanSumArgs::kMaxOut;
-  const int t = threadIdx.x;
-  if (t >= W) return;
   double v = 0.0;
-  for (int p = 0; p < nparts; ++p) v += partial[(size_t)p * W + t];
-  out[t] = v;
+  for (int p = threadIdx.x; p < nparts; p += 32) v += partial[(size_t)p * W + blockIdx.x];
+  v = warp_sum_fixed(v);
+  if (threadIdx.x == 0) out[blockIdx.x] = v;
 }
 
 int grid_for(int64_t n) { return (int)std::min<int64_t>(std::max<int64_t>((n + 255) / 256, 1), 1184); }
@@ -140,7 +139,7 @@ int grid_for(int64_t n) { return (int)std::min<int64_t>(std::max<int64_t>((n + 2
 }  // namespace
 
 void launch_tan_eig(const TanEigArgs& a, int nblocks, cudaStream_t s) {
-  if (nblocks > 0) tan_eig_kernel<<<nblocks, kThreads, 0, s>>>(a);
+  if (nblocks > 0) tan_eig_kernel<<<dim3(nblocks, kEigParts), kThreads, 0, s>>>(a);
 }
 void launch_tan_shift(const double* dlam, int nstates, int gs, double* dE_all, const int* kept_state, int nkept,
                       double* dE_kept, cudaStream_t s) {
@@ -159,8 +158,8 @@ void launch_tan_scale(const double* a, double scale, int64_t n, double* out, cud
 }
 size_t tan_partial_doubles() { return (size_t)kBlocks * TanSumArgs::kMaxOut; }
 void launch_tan_sums(const TanSumArgs& a, double* partial, double* out, cudaStream_t s) {
-  tan_sums_kernel<<<kBlocks, kThreads, 0, s>>>(a, partial);
-  tan_fold_kernel<<<1, 32, 0, s>>>(partial, kBlocks, out);
+  tan_sums_kernel<<<kBlocks, 32, 0, s>>>(a, partial);
+  tan_fold_kernel<<<TanSumArgs::kMaxOut, 32, 0, s>>>(partial, kBlocks, out);
 }
 
 }  // namespace nrg
