@@ -148,6 +148,7 @@ struct nrg_ctx {
   nrg::DevBuf ops_a[6], ops_b[6], opptr;
   nrg::DevBuf dmcnt, dmrec, dmtab;     // Lehmann record counts / offsets, records, frequency tables
   nrg::DevBuf dmtmeta;                 // work items of the tangent Lehmann sums
+  nrg::DevBuf bfac;                    // factors of the back-transformation's reflector groups
   nrg::DevBuf fgtmeta, fgtw;           // lists summed through key bins: tables, sort and moments
   nrg::DevBuf ozw;                     // split-BF16 slices and row scales of the tensor-core products
   cudaEvent_t ev_a[8];
@@ -694,8 +695,24 @@ void run_vectors(nrg_ctx* c, Timer& tm, EigPlan& P, const std::vector<double>& e
   for (int b = 0; b < nb; ++b) { P.yoff[b] = y; y += (int64_t)P.bsize[b] * P.nvec[b]; }
   P.ysize = y;
   if (y == 0) return;
-  std::vector<int> vb, vi, cb, cf, cn, ctab, ctaf;
-  const int bw = backtransform_warps(std::max(P.maxn, 1));
+  std::vector<int> vb, vi, cb, cf, cn, ctab, ctaf, grpb, grpi, grpf(nb, 0);
+  // The back-transformation: blocks up to 900 states by groups of reflectors,
+  // eight vectors per CTA or four while eight leave SMs without a CTA; larger
+  // ones one reflector at a time with two CTAs per SM, which there hides more
+  // than the groups save (one block of 1901 states 17.6 against 22.9 ms; a
+  // two-channel sweep at 300 kept, blocks to about 800 states: 10.0 ms by groups
+  // throughout, 14.9 ms by groups up to 300 states only).
+  const int gmax = std::min(900, backtransform_grouped_max(8));
+  std::vector<int> gtab, gtaf;
+  int gvecs = 0, gmaxn = 1, lmaxn = 1;
+  for (int b = 0; b < nb; ++b) {
+    if (P.nvec[b] == 0) continue;
+    int& m = P.bsize[b] <= gmax ? gmaxn : lmaxn;
+    m = std::max(m, P.bsize[b]);
+    if (P.bsize[b] <= gmax) gvecs += P.nvec[b];
+  }
+  const int gw = gvecs < 8 * c->num_sms ? 4 : 8;
+  const int bw = backtransform_warps(lmaxn);
   for (int b = 0; b < nb; ++b) {
     const int n = P.bsize[b], k = P.nvec[b];
     if (k == 0) continue;
@@ -710,11 +727,19 @@ void run_vectors(nrg_ctx* c, Timer& tm, EigPlan& P, const std::vector<double>& e
       }
     }
     cb.push_back(b); cf.push_back(start); cn.push_back(k - start);
-    for (int x = 0; x < k; x += bw) { ctab.push_back(b); ctaf.push_back(x); }
+    if (n <= gmax) {
+      grpf[b] = (int)grpb.size();
+      for (int q = 0; q < backtransform_groups(n); ++q) { grpb.push_back(b); grpi.push_back(q); }
+      for (int x = 0; x < k; x += gw) { gtab.push_back(b); gtaf.push_back(x); }
+    } else {
+      for (int x = 0; x < k; x += bw) { ctab.push_back(b); ctaf.push_back(x); }
+    }
   }
   Packer pk;
   size_t o_nvec = pk.add(P.nvec), o_yoff = pk.add(P.yoff), o_vb = pk.add(vb), o_vi = pk.add(vi), o_cb = pk.add(cb),
-         o_cf = pk.add(cf), o_cn = pk.add(cn), o_tb = pk.add(ctab), o_tf = pk.add(ctaf);
+         o_cf = pk.add(cf), o_cn = pk.add(cn), o_tb = pk.add(ctab), o_tf = pk.add(ctaf),
+         o_gb = pk.add(gtab), o_gf = pk.add(gtaf), o_pb = pk.add(grpb), o_pi = pk.add(grpi), o_pf = pk.add(grpf);
+  c->bfac.ensure(sizeof(double) * 16 * std::max<size_t>(grpb.size(), 1));
   DevBuf& mb = c->vmeta;
   mb.ensure(pk.host.size() + 256);
   h2d(c, mb.p, pk.host.data(), pk.host.size());
@@ -736,10 +761,21 @@ void run_vectors(nrg_ctx* c, Timer& tm, EigPlan& P, const std::vector<double>& e
   BackArgs ba{};
   ba.bsize = d_bsize; ba.hoff = d_hoff; ba.H_const = c->H.as<double>(); ba.soff = d_soff; ba.tau = c->tau.as<double>();
   ba.nvec = ia.nvec; ba.yoff = ia.yoff; ba.Y = c->Y.as<double>(); ba.Z = c->Z.as<double>(); ba.Zt = c->Zt.as<double>();
-  ba.zoff = ia.yoff; ba.maxn = std::max(P.maxn, 1);
+  ba.zoff = ia.yoff; ba.maxn = lmaxn;
   cudaEvent_t t1 = tm.start();
-  CU(launch_backtransform(ba, (const int*)(base + o_tb), (const int*)(base + o_tf), (int)ctab.size(), c->stream));
-  c->launches++;
+  if (!ctab.empty()) {
+    CU(launch_backtransform(ba, (const int*)(base + o_tb), (const int*)(base + o_tf), (int)ctab.size(), c->stream));
+    c->launches++;
+  }
+  if (!gtab.empty()) {
+    ba.maxn = gmaxn;
+    ba.grp_block = (const int*)(base + o_pb); ba.grp_index = (const int*)(base + o_pi);
+    ba.grp_first = (const int*)(base + o_pf); ba.factors = c->bfac.as<double>();
+    launch_back_factors(ba, (int)grpb.size(), c->stream);
+    CU(launch_backtransform_grouped(ba, (const int*)(base + o_gb), (const int*)(base + o_gf), (int)gtab.size(), gw,
+                                    c->stream));
+    c->launches += 2;
+  }
   tm.stop(t1, &c->timing.backtransform_ms);
   double fl = 0.0;
   for (int b = 0; b < nb; ++b) fl += 2.0 * (double)P.bsize[b] * P.bsize[b] * P.nvec[b];

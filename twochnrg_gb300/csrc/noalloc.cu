@@ -30,14 +30,16 @@ namespace {
 
 constexpr int kN = NRG_NOALLOC_MAX_N;
 // doubles: A copy, Y, five LU arrays, d/e/tau/ev, FP32 copies of d and e
-// (2 kN floats), e^2, the split flags (kN bytes), then an integer area
+// (2 kN floats), e^2, the split flags (kN bytes), then an integer area and the
+// back-transformation's factors
 constexpr size_t kOffA = 0;
 constexpr size_t kOffY = (size_t)kN * kN;
 constexpr size_t kOffLU = 2 * (size_t)kN * kN;
 constexpr size_t kOffVec = 7 * (size_t)kN * kN;
 constexpr size_t kOffInt = kOffVec + 6 * (size_t)kN + (size_t)kN / 8 + 1;
-constexpr size_t kIntWords = 16 + 8 * (size_t)kN;  // in 4-byte words
-constexpr size_t kScratchDoubles = kOffInt + (kIntWords + 1) / 2 + 8;
+constexpr size_t kIntWords = 16 + 9 * (size_t)kN;  // in 4-byte words
+constexpr size_t kOffFac = kOffInt + (kIntWords + 1) / 2 + 8;
+constexpr size_t kScratchDoubles = kOffFac + 4 * (size_t)kN;  // 16 factors per group of four reflectors
 
 static __device__ __align__(256) double g_noalloc_scratch[kScratchDoubles];
 
@@ -48,7 +50,8 @@ struct Layout {
   unsigned char* split;
   int *queue, *flag, *bsize, *soff, *order, *nvec;
   int64_t *hoff, *yoff;
-  int *state_block, *vec_block, *vec_index, *cl_block, *cl_first, *cl_count, *cta_block, *cta_first;
+  int *state_block, *vec_block, *vec_index, *cl_block, *cl_first, *cl_count, *cta_block, *cta_first, *grp_index;
+  double* factors;
 };
 
 Layout layout(double* base) {
@@ -64,6 +67,8 @@ Layout layout(double* base) {
   int* t = ip + 16;
   L.state_block = t; L.vec_block = t + kN; L.vec_index = t + 2 * kN; L.cl_block = t + 3 * kN;
   L.cl_first = t + 4 * kN; L.cl_count = t + 5 * kN; L.cta_block = t + 6 * kN; L.cta_first = t + 7 * kN;
+  L.grp_index = t + 8 * kN;
+  L.factors = base + kOffFac;
   return L;
 }
 
@@ -74,7 +79,7 @@ __global__ void setup_kernel(Layout L, int n, const double* a, int bw) {
   for (int i = tid; i < n * n; i += gridDim.x * blockDim.x) L.A[i] = a[i];
   for (int i = tid; i < n; i += gridDim.x * blockDim.x) {
     L.state_block[i] = 0; L.vec_block[i] = 0; L.vec_index[i] = i;
-    L.cta_block[i] = 0; L.cta_first[i] = i * bw;
+    L.cta_block[i] = 0; L.cta_first[i] = i * bw; L.grp_index[i] = i;
   }
   if (tid == 0) {
     *L.queue = 0; *L.flag = 0; *L.bsize = n; *L.soff = 0; *L.order = 0; *L.nvec = n;
@@ -118,7 +123,7 @@ extern "C" nrg_status nrg_diag_block_noalloc(int n, const double* a, double* eig
   if (tridiag_rows_max_clusters(cl, n < 2 ? 2 : n) <= 0) return NRG_ERR_SIZE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const Layout L = layout(base);
-  const int bw = backtransform_warps(n);
+  const int bw = 4;  // vectors per CTA: at most 64 CTAs either way
   setup_kernel<<<8, 256, 0, s>>>(L, n, a, bw);
   if (cudaGetLastError() != cudaSuccess) return NRG_ERR_CUDA;
   TridiagArgs ta{};
@@ -142,7 +147,11 @@ extern "C" nrg_status nrg_diag_block_noalloc(int n, const double* a, double* eig
   BackArgs ba{};
   ba.bsize = L.bsize; ba.hoff = L.hoff; ba.H_const = L.A; ba.soff = L.soff; ba.tau = L.tau; ba.nvec = L.nvec;
   ba.yoff = L.yoff; ba.Y = L.Y; ba.Z = eigvecs; ba.Zt = nullptr; ba.zoff = L.yoff; ba.maxn = n;
-  if (launch_backtransform(ba, L.cta_block, L.cta_first, (n + bw - 1) / bw, s) != cudaSuccess) return NRG_ERR_CUDA;
+  ba.grp_block = L.cta_block; ba.grp_index = L.grp_index; ba.grp_first = L.cta_block;  // one block: all 0
+  ba.factors = L.factors;
+  launch_back_factors(ba, backtransform_groups(n), s);
+  if (launch_backtransform_grouped(ba, L.cta_block, L.cta_first, (n + bw - 1) / bw, bw, s) != cudaSuccess)
+    return NRG_ERR_CUDA;
   if (cudaMemcpyAsync(eigvals, L.ev, sizeof(double) * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
     return NRG_ERR_CUDA;
   int flag = 0;

@@ -242,7 +242,21 @@ struct BackArgs {
   double* Zt;             // transposed (n x nvec) at zoff, may be null
   const int64_t* zoff;
   int maxn;
+  // the grouped kernel: groups of kBackGroup reflectors, their triangular
+  // factors (16 doubles per group) and each block's first group
+  const int* grp_block;
+  const int* grp_index;
+  const int* grp_first;   // [blocks]
+  double* factors;
 };
+// Blocks up to backtransform_grouped_max(warps) states fit the grouped kernel
+// (groups of reflectors) with that many vectors per CTA.
+constexpr int kBackGroup = 4;
+int backtransform_grouped_max(int warps);
+int backtransform_groups(int n);    // groups of an n-state block
+void launch_back_factors(const BackArgs& a, int ngroups, cudaStream_t s);
+cudaError_t launch_backtransform_grouped(const BackArgs& a, const int* cta_block, const int* cta_first, int nctas,
+                                         int warps, cudaStream_t s);
 cudaError_t launch_backtransform(const BackArgs& a, const int* cta_block, const int* cta_first, int nctas,
                                  cudaStream_t s);
 size_t backtransform_smem_bytes(int maxn);
