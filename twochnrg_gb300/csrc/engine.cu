@@ -23,6 +23,7 @@
 #include <stdexcept>
 #include <string>
 #include <atomic>
+#include <limits>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -87,6 +88,18 @@ struct OpMeta {
     for (size_t k = 0; k < bi.size(); ++k) if (bi[k] == i && bj[k] == j) return (int)k;
     return -1;
   }
+};
+
+// OpMeta::find by a table, for the loops over all segment pairs of a plan.
+struct PairIndex {
+  int n = 0;
+  std::vector<int> at;
+  explicit PairIndex(const OpMeta& m) {
+    for (size_t k = 0; k < m.bi.size(); ++k) n = std::max({n, m.bi[k] + 1, m.bj[k] + 1});
+    at.assign((size_t)n * n, -1);
+    for (size_t k = m.bi.size(); k-- > 0;) at[(size_t)m.bi[k] * n + m.bj[k]] = (int)k;  // the first of equal pairs
+  }
+  int find(int i, int j) const { return i < 0 || j < 0 || i >= n || j >= n ? -1 : at[(size_t)i * n + j]; }
 };
 
 struct DmTan { static constexpr int NP = 4; };  // parameter directions of the DM-NRG tangents
@@ -882,6 +895,8 @@ AsmTables prepare_assembly(nrg_ctx* c, const ModelSpec& m, const Basis& B, const
   std::vector<int> nseg(nb);
   std::vector<int64_t> pair_base(nb), pair_fwd, pair_bwd;
   std::vector<int> pair_fwd_ld, pair_bwd_ld;
+  std::vector<PairIndex> old_index;
+  for (int o = 0; o < nops_h; ++o) old_index.emplace_back(oldops[o]);
   for (int b = 0; b < nb; ++b) {
     const auto& sg = B.seg[b];
     nseg[b] = (int)sg.size();
@@ -890,8 +905,8 @@ AsmTables prepare_assembly(nrg_ctx* c, const ModelSpec& m, const Basis& B, const
       for (size_t q = 0; q < sg.size(); ++q)
         for (int o = 0; o < nops_h; ++o) {
           const OpMeta& om = oldops[o];
-          int kf = om.find(ob(sg[p].old_block), ob(sg[q].old_block));
-          int kb = om.find(ob(sg[q].old_block), ob(sg[p].old_block));
+          const int kf = old_index[o].find(ob(sg[p].old_block), ob(sg[q].old_block));
+          const int kb = old_index[o].find(ob(sg[q].old_block), ob(sg[p].old_block));
           pair_fwd.push_back(kf >= 0 ? om.off[kf] : -1);
           pair_fwd_ld.push_back(kf >= 0 ? old_size[om.bj[kf]] : 0);
           pair_bwd.push_back(kb >= 0 ? om.off[kb] : -1);
@@ -989,8 +1004,14 @@ void plan_update(UpdatePlan& U, const ModelSpec& m, const Basis& B, const EigPla
   const int nops = (int)m.op_kind.size();
   U.newops.assign(nops, OpMeta());
   const int nk = K.blk.nblocks();
+  // The site factors depend on the two spins and the two site states only and
+  // most block pairs share them: one evaluation per plan.
+  const int NT = m.site.nstates;
+  std::map<std::pair<double, double>, std::vector<double>> factors;  // of one operator; NaN: not yet evaluated
   for (int o = 0; o < nops; ++o) {
     OpMeta& no = U.newops[o];
+    const PairIndex old_index(o < (int)oldops.size() ? oldops[o] : OpMeta());
+    factors.clear();
     for (int i = 0; i < nk; ++i)
       for (int j = 0; j < nk; ++j) {
         if (!op_check(m, m.op_check[o], K.blk, i, j)) continue;
@@ -1008,6 +1029,13 @@ void plan_update(UpdatePlan& U, const ModelSpec& m, const Basis& B, const EigPla
         const int jid = (int)U.jobs.size();
         U.jobs.push_back(J);
         const double SI = B.blk.q(bI, 1), SJ = B.blk.q(bJ, 1);
+        std::vector<double>& known = factors[{SI, SJ}];
+        if (known.empty()) known.assign((size_t)NT * NT, std::numeric_limits<double>::quiet_NaN());
+        auto site_factor = [&](int ti, int tj) {
+          double& g = known[(size_t)ti * NT + tj];
+          if (std::isnan(g)) g = op_site_factor(m, m.op_kind[o], SI, SJ, ti, tj);
+          return g;
+        };
         const auto& segI = B.seg[bI];
         const auto& segJ = B.seg[bJ];
         for (const Segment& p : segI)
@@ -1026,17 +1054,17 @@ void plan_update(UpdatePlan& U, const ModelSpec& m, const Basis& B, const EigPla
                   if (m.op_kind[o] == OP_IMPONLY) {
                     if (tu_ != tv) continue;
                   } else {
-                    g = op_site_factor(m, m.op_kind[o], SI, SJ, tu_, tv);
+                    g = site_factor(tu_, tv);
                     if (g == 0.0) continue;
                   }
                   const OpMeta& om = oldops[o];
-                  int kx = om.find(ob(p.old_block), ob(q.old_block));
+                  const int kx = old_index.find(ob(p.old_block), ob(q.old_block));
                   if (kx < 0) continue;
                   G.mode = 1; G.coef = g; G.old_off = om.off[kx]; G.op = o;
                   G.old_ld = opsize ? (*opsize)[ob(q.old_block)] : q.count;
                 } else {
                   if (p.old_block != q.old_block) continue;
-                  double g = op_site_factor(m, m.op_kind[o], SI, SJ, tu_, tv);
+                  double g = site_factor(tu_, tv);
                   if (g == 0.0) continue;
                   G.mode = 0; G.coef = g;
                 }

@@ -3,7 +3,7 @@
 
 #include <algorithm>
 #include <cmath>
-#include <mutex>
+#include <cstdint>
 #include <stdexcept>
 
 namespace nrg {
@@ -46,6 +46,7 @@ double fd_onechS(int sigma, int ti, int tj) {
 struct TwoChTables {
   double fd[2][2][16][16];  // [ch-1][sigma==+1][ti][tj]
   double spsm[16][16];      // TwoChQS_SpSm_table (:140-185)
+  bool pair[2][2][16][16];
   TwoChTables() {
     for (auto& a : fd) for (auto& b : a) for (auto& c : b) for (double& x : c) x = 0.0;
     const double r = 1.0 / std::sqrt(2.0), mr = -1.0 / std::sqrt(2.0);
@@ -61,7 +62,19 @@ struct TwoChTables {
     for (int i = 0; i < 16; ++i) for (int j = 0; j < 16; ++j) spsm[i][j] = (i == j) ? 1.0 : 0.0;
     const int pairs[][2] = {{1, 3}, {2, 4}, {11, 13}, {12, 14}, {8, 9}, {9, 10}, {8, 10}};
     for (auto& p : pairs) { spsm[p[0]][p[1]] = 1.0; spsm[p[1]][p[0]] = 1.0; }
+    for (int c = 0; c < 2; ++c)
+      for (int s = 0; s < 2; ++s)
+        for (int tp = 0; tp < 16; ++tp)
+          for (int t = 0; t < 16; ++t) {
+            pair[c][s][tp][t] = false;
+            for (int i = 0; i < 16; ++i)
+              for (int j = 0; j < 16; ++j)
+                if (fd[c][s][i][j] != 0.0 && spsm[i][tp] != 0.0 && spsm[j][t] != 0.0) pair[c][s][tp][t] = true;
+          }
   }
+  // Whether any pair of site states of the two states' multiplets is connected
+  // by f^dagger: if not, the sums over the members vanish term by term.
+  bool couples(int ch, int sigma, int tp, int t) const { return pair[ch - 1][sigma == 1][tp][t]; }
   double f(int ch, int sigma, int ti, int tj) const {
     if (ti < 0 || tj < 0 || ti > 15 || tj > 15 || (ch != 1 && ch != 2) || (sigma != 1 && sigma != -1)) return 0.0;
     return fd[ch - 1][sigma == 1][ti][tj];
@@ -99,21 +112,28 @@ double clebsch(double J1, double M1, double J2, double M2, double J, double M) {
 }
 
 namespace {
-// Memoised Clebsch-Gordan: pure function of six half-integers.  Shared by
-// the host threads of batched sweeps, hence the lock.
+// Clebsch-Gordan coefficients as a function of six half-integers, kept in a
+// table of the calling thread: the key packs 2a .. 2f, and a new coefficient
+// takes its slot from the old one (64 KB per thread; a full-size two-channel
+// sweep meets a few thousand).  The tables ask for the same few coefficients
+// hundreds of thousands of times in a sweep; a tree of all threads behind a lock
+// took 9.6 of a 45 ms pair of chain sweeps, with both threads waiting for it.
 double cg(double a, double b, double c, double d, double e, double f) {
-  static std::map<std::array<double, 6>, double> memo;
-  static std::mutex mu;
-  std::array<double, 6> k{a, b, c, d, e, f};
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = memo.find(k);
-    if (it != memo.end()) return it->second;
+  struct Slot { uint64_t key; double v; };
+  constexpr int kBits = 12;
+  thread_local std::vector<Slot> table((size_t)1 << kBits, Slot{~uint64_t(0), 0.0});
+  const double q[6] = {a, b, c, d, e, f};
+  uint64_t key = 0;
+  for (double x : q) {
+    const double t = 2.0 * x + 512.0;  // 10 bits each
+    if (!(t >= 0.0 && t < 1024.0)) return clebsch(a, b, c, d, e, f);
+    const int i = (int)t;
+    if ((double)i != t) return clebsch(a, b, c, d, e, f);
+    key = key << 10 | (uint64_t)i;
   }
-  double v = clebsch(a, b, c, d, e, f);
-  std::lock_guard<std::mutex> lock(mu);
-  memo.emplace(k, v);
-  return v;
+  Slot& s = table[(key * 0x9e3779b97f4a7c15ull) >> (64 - kBits)];
+  if (s.key != key) s = Slot{key, clebsch(a, b, c, d, e, f)};
+  return s.v;
 }
 }  // namespace
 
@@ -521,10 +541,11 @@ double hn_coef_1chQS(const Site& st, double Si, int typep, int type) {
       double Szcf = Si - Sz, Szcfp = Szcf - dS, Szp = Sz + dS;
       qp[2] = Sz + dS;
       int sstp = ss.find(qp);
+      const double a3 = fd_onech(sigma, sstp, sst);
+      if (a3 == 0.0) continue;
       double a0 = cg(Scf, Szcf, Stt, Sz, Si, Si);
       double a1 = cg(Scfp, Szcfp, Stp, Szp, Si, Si);
       double a2 = cg(Scfp, Szcfp, 0.5, dS, Scf, Szcf);
-      double a3 = fd_onech(sigma, sstp, sst);
       coef += a0 * a1 * a2 * a3;
     }
   }
@@ -536,6 +557,7 @@ double hn_coef_1chQS(const Site& st, double Si, int typep, int type) {
 double hn_full_2chQS(const Site& st, double Si, int typep, int type, int ich, int sigma) {
   const BlockArray& ss = st.blk;
   const TwoChTables& T = twoch();
+  if (!T.couples(ich, sigma, typep, type)) return 0.0;
   int bp = st.block_of_state(typep), b = st.block_of_state(type);
   double Stp = ss.q(bp, 1), Sztp = ss.q(bp, 2), Stt = ss.q(b, 1), Szt = ss.q(b, 2);
   double Soldp = Si - Sztp, Sold = Si - Szt;
@@ -791,7 +813,7 @@ double op_site_factor(const ModelSpec& m, int op, double Si, double Sj, int ti, 
     int sigma = 0; double norm = 1.0;
     if (!deq(c0, 0.0)) { sigma = -1; norm = c0; }
     else if (!deq(c1, 0.0)) { sigma = 1; norm = c1; }
-    if (sigma == 0) return 0.0;
+    if (sigma == 0 || !T.couples(ich, sigma, tj, ti)) return 0.0;
     double acc = 0.0;
     for (double Szcfj = Scfj; Szcfj >= -Scfj; Szcfj -= 1.0) {
       double Szi = Si - Szcfj, Szj = Sj - Szcfj;
