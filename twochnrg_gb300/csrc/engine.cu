@@ -172,8 +172,9 @@ struct nrg_ctx {
   cudaEvent_t fork = nullptr, join[kMaxSplit] = {};
   // the row kernel beside the cluster kernel of the middle blocks
   cudaStream_t rows_stream = nullptr;
+  cudaEvent_t span_join = nullptr;
   cudaEvent_t rows_fork = nullptr, rows_join = nullptr;
-  nrg::DevBuf gpart_k[kMaxSplit], gbig;
+  nrg::DevBuf gpart_k[kMaxSplit], gbig, rlist, slist, swork;
   // mixed precision: per concurrent grid the blocked reduction's [V W], column
   // and share scratch, and the tensor-core product's slices
   nrg::DevBuf pvw[kMaxSplit], pcol[kMaxSplit], ppart[kMaxSplit], ozk[kMaxSplit];
@@ -261,9 +262,9 @@ struct Timer {
 };
 
 // Stream-ordered copies that also count the bytes crossing the host boundary.
-void h2d(nrg_ctx* c, void* dst, const void* src, size_t bytes) {
+void h2d(nrg_ctx* c, void* dst, const void* src, size_t bytes, cudaStream_t s = nullptr) {
   if (!bytes) return;
-  CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream));
+  CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s ? s : c->stream));
   c->timing.h2d_bytes += (int64_t)bytes;
 }
 void d2h(nrg_ctx* c, void* dst, const void* src, size_t bytes) {
@@ -366,8 +367,8 @@ int choose_rows_cluster(int maxn) {
 }
 
 // Blocks at least this large are tridiagonalized by a cooperative grid of
-// many SMs (one block after the other per grid); smaller ones by one
-// thread-block cluster each.
+// many SMs (one block after the other per grid) where contexts share the GPU
+// or in the mixed form; a context alone decides by the estimates at plan_span.
 int big_block_threshold() {
   const char* s = std::getenv("NRG_BIG_N");
   return s ? std::atoi(s) : 1800;
@@ -510,6 +511,74 @@ std::vector<std::vector<int>> deal_by_cost(const std::vector<int>& blocks, const
   return bins;
 }
 
+// The span kernel's share of the blocks (k_span.cu).  From 450 states on a block
+// may go to it (a two-channel sweep at 300 kept 107 ms, 117 with only the blocks
+// that do not fit the row kernel); smaller ones are faster in the row kernel
+// (450 states: 2.9 us per column of a group's latency against 2.2).
+int span_from() {
+  const char* s = std::getenv("NRG_SPAN_N");
+  return s ? std::atoi(s) : 450;
+}
+constexpr int kSpanCopies = 4;     // of its exchange area (1901 states on 152 CTAs: 28.4 ms with 1, 26.7 with 4)
+constexpr int kGridFrom = 1200;    // smallest block considered for the whole-GPU kernel beside span groups
+
+// Times of one block in us, within 20 % of those measured: in the row kernel on a
+// cluster of 16 (64 to 600 states), in the span kernel on a group of G CTAs (640
+// to 3400 states on 16 to 152 CTAs; the last factor for rows that stay in L2),
+// and in the grid kernel as one of K grids that share the GPU (1900 to 3400).
+double rows_cost(int n) { return n * (2.2 + (double)n * n / 47e3); }
+double span_cost(int n, int G) {
+  const double n2 = (double)n * n, in_l2 = std::max(0.0, 1.0 - 180e3 * G / (8.0 * n2));
+  return n * (3.6 + n / 840.0 + n2 / (3230.0 * G) * (1.0 + 0.6 * std::min(1.0, 2.0 * in_l2)));
+}
+double grid_cost(int n, int K) { return n * (23.5 - 2.2 * std::min(K, 4) + 1.6e-6 * K * (double)n * n); }
+
+// Blocks (largest first) to k bins, each to the least loaded one; returns the
+// largest load.
+double deal_greedy(const std::vector<double>& cost, size_t from, size_t to, int k, std::vector<int>* bin) {
+  std::vector<double> load(k, 0.0);
+  if (bin) bin->assign(to - from, 0);
+  for (size_t i = from; i < to; ++i) {
+    const int q = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+    load[q] += cost[i];
+    if (bin) (*bin)[i - from] = q;
+  }
+  return *std::max_element(load.begin(), load.end());
+}
+
+// How many of the blocks (largest first) go to the span kernel, in how many
+// groups of G CTAs, beside how many clusters of the row kernel.
+struct SpanPlan { int n = 0, G = 0, groups = 0, rows_clusters = 0; double time = 0.0; };
+
+// Of sizes[from ..] (largest first), sizes[from .. must) do not fit the row kernel.
+// sms SMs, of which the row kernel's clusters of 16 can use 16 * rmax at one CTA
+// per SM.
+SpanPlan plan_span(const std::vector<int>& all_sizes, int from, int all_must, int sms, int rmax) {
+  const std::vector<int> sizes(all_sizes.begin() + from, all_sizes.end());
+  const int nb = (int)sizes.size(), must = all_must - from;
+  if (nb == 0) return SpanPlan();
+  std::vector<double> rc(nb), sc(nb);
+  for (int i = must; i < nb; ++i) rc[i] = rows_cost(sizes[i]);
+  SpanPlan best;
+  double t = must > 0 || rmax < 1 ? 1e300 : deal_greedy(rc, 0, nb, rmax, nullptr);
+  best.time = t;
+  for (int s = std::max(must, 1); s <= nb && s <= must + 6; ++s) {
+    if (s > must && sizes[s - 1] < std::max(3, span_from())) break;
+    for (int r = s < nb ? 1 : 0; r <= (s < nb ? rmax : 0); ++r) {
+      const double tr = r > 0 ? deal_greedy(rc, s, nb, r, nullptr) : 0.0;
+      for (int k = 1; k <= s && k <= 8; ++k) {
+        if (sms - 16 * r < 16 * k) break;
+        const int G = (sms - 16 * r) / k;
+        if (G < 16) break;
+        for (int i = 0; i < s; ++i) sc[i] = span_cost(sizes[i], G);
+        const double tt = std::max(tr, deal_greedy(sc, 0, s, k, nullptr)) + 20.0;
+        if (tt < t) { t = best.time = tt; best.n = s; best.G = G; best.groups = k; best.rows_clusters = r; }
+      }
+    }
+  }
+  return best;
+}
+
 // `order`: all blocks, largest first (host copy `order_h`); the big blocks
 // form its prefix.
 void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::vector<int>& order_h,
@@ -525,6 +594,42 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
   ta.nblocks = nb; ta.order = d_order; ta.bsize = d_bsize; ta.hoff = d_hoff; ta.soff = d_soff;
   ta.H = c->H.as<double>(); ta.d = c->d.as<double>(); ta.e = c->e.as<double>(); ta.tau = c->tau.as<double>();
   ta.queue = c->red.as<int>(); ta.flag = c->flag.as<int>(); ta.maxn = std::max(P.maxn, 2);
+  // Who takes which blocks.  A context that shares the GPU with others (batch
+  // workers) keeps to kernels that need no co-resident grid, so that the contexts
+  // need not wait for each other: whole-GPU grids for the largest blocks only,
+  // the cluster kernel for the middle ones.  Alone, the largest blocks go to
+  // concurrent whole-GPU grids (4 FMA per element of a triangle, 15 to 21 us per
+  // column of latency) and after them the others to span groups (6, but 4 to 7 us)
+  // beside the row kernel, split where the sum of both is smallest: 2600 states
+  // 74 ms by the span kernel, 84 by the grid; 3400 states 160 and 138; two / three
+  // blocks of 1900 52 / 70 ms and 56 / 64; eight of 1200 42 ms (cluster kernel 86).
+  SpanPlan sp;
+  const bool cluster_only = std::getenv("NRG_CLUSTER") || std::getenv("NRG_CLUSTER_THREADS");
+  if (!c->shared_gpu && !cluster_only && !(mixed && nbig > 0) && nb > 0 && P.bsize[order_h[0]] > span_from()) {
+    std::vector<int> sizes(nb);
+    int must = 0;
+    for (int q = 0; q < nb; ++q) sizes[q] = P.bsize[order_h[q]];
+    while (must < nb && sizes[must] > std::max(2, rows_block_threshold())) ++must;
+    const int rmax = tridiag_span_max_ctas(16) / 16;
+    const bool forced = std::getenv("NRG_BIG_N") != nullptr;  // nbig stays
+    double best = 1e300;
+    const int k0 = forced ? nbig : 0;
+    int pick = nbig;
+    for (int k = k0; k <= must && (forced ? k == nbig : k == 0 || sizes[k - 1] >= kGridFrom); ++k) {
+      double t = 0.0;
+      if (k > 0) {
+        std::vector<double> gc(k);
+        const int K = grid_split(k);
+        for (int q = 0; q < k; ++q) gc[q] = grid_cost(sizes[q], K);
+        t = deal_greedy(gc, 0, k, K, nullptr);
+      }
+      const bool fits = k == nb || tridiag_span_fits(sizes[k]);
+      const SpanPlan p = fits ? plan_span(sizes, k, must, c->num_sms, rmax) : SpanPlan();
+      if (fits && t + p.time < best) { best = t + p.time; sp = p; pick = k; }
+    }
+    nbig = pick;
+  }
+  const int nspan = sp.n;
   const int K = nbig > 0 ? grid_split(nbig) : 0;
   std::vector<std::vector<int>> bins(std::max(K, 1));
   size_t o_bins[nrg_ctx::kMaxSplit] = {};
@@ -543,8 +648,28 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
     c->gbig.ensure(pk.host.size() + 256);
     h2d(c, c->gbig.p, pk.host.data(), pk.host.size());
   }
+  size_t o_span = 0, o_sfirst = 0;
+  if (nspan > 0) {
+    std::vector<int> span_list, span_first;
+    std::vector<double> cst(nspan);
+    for (int q = 0; q < nspan; ++q) cst[q] = span_cost(P.bsize[order_h[nbig + q]], sp.G);
+    std::vector<int> bin;
+    deal_greedy(cst, 0, nspan, sp.groups, &bin);
+    for (int k = 0; k < sp.groups; ++k) {
+      span_first.push_back((int)span_list.size());
+      for (int q = 0; q < nspan; ++q)
+        if (bin[q] == k) span_list.push_back(order_h[nbig + q]);
+    }
+    span_first.push_back(nspan);
+    Packer pk;
+    o_span = pk.add(span_list); o_sfirst = pk.add(span_first);
+    c->slist.ensure(pk.host.size() + 256);
+    h2d(c, c->slist.p, pk.host.data(), pk.host.size());
+    c->swork.ensure(sizeof(double) * tridiag_span_work(P.bsize[order_h[nbig]], sp.groups, sp.G, kSpanCopies));
+    if (!c->span_join) CU(cudaEventCreateWithFlags(&c->span_join, cudaEventDisableTiming));
+  }
   std::unique_lock<std::mutex> coop(g_coop_mu, std::defer_lock);
-  if (K >= 1) {
+  if (K >= 1 || nspan > 0) {
     coop.lock();
     for (int k = 0; k < K; ++k)
       if (!c->join[k]) CU(cudaEventCreateWithFlags(&c->join[k], cudaEventDisableTiming));
@@ -626,7 +751,7 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
   }
   // The other blocks: the middle ones by the cluster kernel, those whose rows
   // fit in a cluster's shared memory by the row kernel beside it.
-  int nrows0 = nbig, rcl = 0, rncl = 0;
+  int nrows0 = nbig + nspan, rcl = 0, rncl = 0;
   while (nrows0 < nb && P.bsize[order_h[nrows0]] > rows_block_threshold()) ++nrows0;
   for (; nrows0 < nb; ++nrows0) {
     const int maxs = std::max(P.bsize[order_h[nrows0]], 2);
@@ -635,7 +760,10 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
     for (; rncl <= 0 && rcl < 16; ) { rcl *= 2; rncl = tridiag_rows_max_clusters(rcl, maxs); }
     if (rncl > 0) break;
   }
-  const bool both = nbig < nrows0 && nrows0 < nb;
+  const int nmid = nrows0 - nbig - nspan;
+  if (nspan > 0)  // two cooperative kernels at once might each get part of the SMs
+    for (int k = 0; K > 1 && k < K; ++k) CU(cudaStreamWaitEvent(c->stream, c->join[k], 0));
+  const bool both = nspan + nmid > 0 && nrows0 < nb;
   if (both) {
     if (!c->rows_stream) {
       CU(cudaStreamCreateWithFlags(&c->rows_stream, cudaStreamNonBlocking));
@@ -643,39 +771,72 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
       CU(cudaEventCreateWithFlags(&c->rows_join, cudaEventDisableTiming));
     }
     CU(cudaEventRecord(c->rows_fork, c->stream));
+    CU(cudaStreamWaitEvent(c->rows_stream, c->rows_fork, 0));
   }
-  if (nbig < nrows0) {
-    int maxs = P.bsize[order_h[nbig]];
+  auto launch_rows = [&](cudaStream_t s) {
     TridiagArgs ts = ta;
-    ts.order = d_order + nbig;
-    ts.nblocks = nrows0 - nbig;
+    const int k = std::min({rncl, nb - nrows0, nspan > 0 ? std::max(1, sp.rows_clusters) : rncl});
+    std::vector<double> cst(nb);
+    std::vector<int> bin, list, first;
+    for (int q = nrows0; q < nb; ++q) cst[q] = rows_cost(P.bsize[order_h[q]]);
+    deal_greedy(cst, nrows0, nb, k, &bin);
+    for (int q = 0; q < k; ++q) {
+      first.push_back((int)list.size());
+      for (int i = nrows0; i < nb; ++i)
+        if (bin[i - nrows0] == q) list.push_back(order_h[i]);
+    }
+    first.push_back((int)list.size());
+    Packer pk;
+    const size_t o_list = pk.add(list), o_first = pk.add(first);
+    c->rlist.ensure(pk.host.size() + 256);
+    h2d(c, c->rlist.p, pk.host.data(), pk.host.size(), s);
+    ts.order = (const int*)(c->rlist.as<char>() + o_list); ts.first = (const int*)(c->rlist.as<char>() + o_first);
+    ts.nblocks = nb - nrows0;
+    ts.maxn = std::max(P.bsize[order_h[nrows0]], 2);
+    CU(launch_tridiag_rows(ts, rcl, k, s));
+    c->launches++; c->timing.tridiag_launches++;
+  };
+  // Beside the span kernel the row kernel goes first: its clusters of 16 need SMs
+  // of one GPC, the span kernel's CTAs take what they leave.
+  if (nspan > 0) {
+    cudaStream_t ss = both ? c->rows_stream : c->stream;
+    if (both) launch_rows(c->stream);
+    SpanArgs sa{};
+    sa.list = (const int*)(c->slist.as<char>() + o_span); sa.first = (const int*)(c->slist.as<char>() + o_sfirst);
+    sa.work = c->swork.as<double>(); sa.G = sp.G; sa.copies = kSpanCopies;
+    TridiagArgs ts = ta;
+    ts.maxn = P.bsize[order_h[nbig]];
+    CU(launch_tridiag_span(ts, sa, sp.groups, ss));
+    c->launches++; c->timing.tridiag_launches++;
+    CU(cudaEventRecord(c->span_join, ss));
+    CU(cudaStreamWaitEvent(c->stream, c->span_join, 0));
+  }
+  if (nmid > 0) {
+    int maxs = P.bsize[order_h[nbig + nspan]];
+    TridiagArgs ts = ta;
+    ts.order = d_order + nbig + nspan;
+    ts.nblocks = nmid;
     ts.maxn = std::max(maxs, 2);
     int cluster = choose_cluster(maxs, c->shared_gpu);
     int threads = cluster_threads(c->shared_gpu);
     int ncl = tridiag_max_clusters(cluster, ts.maxn, threads);
     if (ncl <= 0) { cluster = 8; threads = 512; ncl = tridiag_max_clusters(cluster, ts.maxn, threads); }
     if (ncl <= 0) throw NrgError(NRG_ERR_SIZE, "tridiagonalization does not fit on the device");
-    ncl = std::min(ncl, nrows0 - nbig);
+    ncl = std::min(ncl, nmid);
     CU(launch_tridiag(ts, cluster, ncl, c->stream, threads));
     c->launches++; c->timing.tridiag_launches++;
   }
-  if (nrows0 < nb) {
-    cudaStream_t sr = both ? c->rows_stream : c->stream;
-    if (both) CU(cudaStreamWaitEvent(sr, c->rows_fork, 0));
-    TridiagArgs ts = ta;
-    ts.order = d_order + nrows0;
-    ts.nblocks = nb - nrows0;
-    ts.maxn = std::max(P.bsize[order_h[nrows0]], 2);
-    CU(launch_tridiag_rows(ts, rcl, std::min(rncl, nb - nrows0), sr));
-    c->launches++; c->timing.tridiag_launches++;
+  if (nspan == 0 && nrows0 < nb) {
+    launch_rows(both ? c->rows_stream : c->stream);
     if (both) {
-      CU(cudaEventRecord(c->rows_join, sr));
+      CU(cudaEventRecord(c->rows_join, c->rows_stream));
       CU(cudaStreamWaitEvent(c->stream, c->rows_join, 0));
     }
   }
   for (int k = 0; K > 1 && k < K; ++k) CU(cudaStreamWaitEvent(c->stream, c->join[k], 0));
   if (coop.owns_lock()) {
     for (int k = 0; k < K; ++k) CU(cudaEventSynchronize(c->join[k]));
+    if (nspan > 0) CU(cudaEventSynchronize(c->span_join));
     coop.unlock();
   }
   tm.stop(t0, &c->timing.tridiag_ms);
@@ -3241,6 +3402,7 @@ void nrg_destroy(nrg_ctx* ctx) {
   if (ctx->rows_stream) { cudaStreamSynchronize(ctx->rows_stream); cudaStreamDestroy(ctx->rows_stream); }
   if (ctx->rows_fork) cudaEventDestroy(ctx->rows_fork);
   if (ctx->rows_join) cudaEventDestroy(ctx->rows_join);
+  if (ctx->span_join) cudaEventDestroy(ctx->span_join);
   if (ctx->bsync) cudaEventDestroy(ctx->bsync);
   cudaStreamDestroy(ctx->stream);
   delete ctx->tan;

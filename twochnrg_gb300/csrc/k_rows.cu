@@ -89,28 +89,6 @@ __device__ __forceinline__ bool try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Sums of RT values over the warp's lanes in RT + log2(32 / RT) additions: the
-// lanes halve the set of values they carry at each of the first steps.  Lane
-// l with l % (32 / RT) == 0 ends with value l / (32 / RT).
-template <int RT>
-__device__ __forceinline__ double reduce_rows(double* a) {
-  const int lane = threadIdx.x & 31;
-  int o = 16;
-#pragma unroll
-  for (int h = RT / 2; h >= 1; h >>= 1) {
-    const bool up = (lane & o) != 0;
-#pragma unroll
-    for (int q = 0; q < h; ++q) {
-      const double send = up ? a[q] : a[q + h], keep = up ? a[q + h] : a[q];
-      a[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-    }
-    o >>= 1;
-  }
-  double v = a[0];
-  for (; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
 struct RowsSm {
   double* x;      // 2 x ldv: u of the last step, x of this one
   double* w;
@@ -244,12 +222,10 @@ __global__ void __launch_bounds__(kRowsThreads, 3) tridiag_rows_kernel(TridiagAr
   // Steps done over all blocks: step g uses mbarrier g & 1 in its phase g >> 1.
   uint32_t g = 0;
 
-  // The blocks (largest first) are dealt to the clusters in a snake, so that
-  // every CTA of a cluster knows its blocks without asking another.
-  const int ncl = (int)gridDim.x / CL, me = (int)blockIdx.x / CL;
-  for (int q = 0; q * ncl < A.nblocks; ++q) {
-    const int qi = q * ncl + ((q & 1) ? ncl - 1 - me : me);
-    if (qi >= A.nblocks) continue;
+  // Every cluster has its list of blocks, so that its CTAs need not ask another
+  // for the next one.
+  const int me = (int)blockIdx.x / CL, q1 = A.first ? A.first[me + 1] : A.nblocks;
+  for (int qi = A.first ? A.first[me] : 0; qi < q1; ++qi) {
     const int b = A.order[qi];
     const int n = A.bsize[b];
     double* H = A.H + A.hoff[b];

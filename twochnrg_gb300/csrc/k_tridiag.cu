@@ -10,7 +10,9 @@
 // algorithmic count (a full-storage update does n^3).  The shared sweep is
 // lower_sweep below; the kernels differ in who cooperates on a block:
 //   tridiag_kernel       one thread-block CLUSTER per block (blocks pulled
-//                        largest first from a work counter); the CTAs' shares
+//                        largest first from a work counter), for blocks past
+//                        the row kernel's size in contexts that share the GPU
+//                        (a context alone has k_span.cu); the CTAs' shares
 //                        of y are summed through distributed shared memory
 //                        after one hardware cluster barrier per step;
 //   tridiag_grid_kernel  every CTA of a cooperative grid on the same block

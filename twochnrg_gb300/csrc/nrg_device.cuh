@@ -61,6 +61,28 @@ __device__ __forceinline__ double warp_sum_fixed(double v) {
   if (en >= 0x7ff) return __hiloint2double((hi & 0x80000000) | 0x7ff00000, 0);
   return __hiloint2double(hi + (sc << 20), __double2loint(d));
 }
+
+// Sums of RT values over the warp's lanes in RT + log2(32 / RT) additions: the
+// lanes halve the set of values they carry at each of the first steps.  Lane
+// l with l % (32 / RT) == 0 ends with value l / (32 / RT).
+template <int RT>
+__device__ __forceinline__ double reduce_rows(double* a) {
+  const int lane = threadIdx.x & 31;
+  int o = 16;
+#pragma unroll
+  for (int h = RT / 2; h >= 1; h >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int q = 0; q < h; ++q) {
+      const double send = up ? a[q] : a[q + h], keep = up ? a[q + h] : a[q];
+      a[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+    o >>= 1;
+  }
+  double v = a[0];
+  for (; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
 #endif
 
 // Error flags a kernel can raise without trapping; the host reads the word
@@ -172,6 +194,8 @@ struct TridiagArgs {
   double* d;
   double* e;
   double* tau;
+  const int* first;      // launch_tridiag_rows: cluster q's blocks are order[first[q]] .. order[first[q + 1] - 1]
+                         // (NULL: one cluster, all blocks)
   int* queue;            // work counter (reset to 0 before launch)
   int* flag;
   int maxn;
@@ -181,6 +205,22 @@ cudaError_t launch_tridiag(const TridiagArgs& a, int cluster, int nclusters, cud
 size_t tridiag_smem_bytes(int maxn, int cluster, int threads = 512);
 int tridiag_max_clusters(int cluster, int maxn, int threads = 512);
 // Blocks whose rows fit in a cluster's shared memory (k_rows.cu).
+// One block per group of G CTAs, the groups' blocks in list[first[g]] ..
+// list[first[g + 1]) (k_span.cu).  A cooperative launch; work:
+// tridiag_span_work(maxn, groups, G) doubles.
+struct SpanArgs {
+  const int* list;
+  const int* first;
+  double* work;
+  int G;
+  int copies;        // of the exchange area, each read by every copies-th CTA (up to 32)
+  bool clusters;     // launch as clusters of 16 (G a multiple of 16)
+  int smem_doubles;  // set by the launch
+};
+size_t tridiag_span_work(int maxn, int groups, int G, int copies);
+bool tridiag_span_fits(int n);        // its vectors fit in shared memory
+int tridiag_span_max_ctas(int maxn);  // that can be resident in clusters of 16; 0: does not fit
+cudaError_t launch_tridiag_span(const TridiagArgs& a, SpanArgs p, int groups, cudaStream_t s);
 size_t tridiag_rows_smem_bytes(int maxn, int cluster);
 int tridiag_rows_max_clusters(int cluster, int maxn);
 cudaError_t launch_tridiag_rows(const TridiagArgs& a, int cluster, int nclusters, cudaStream_t s);
