@@ -1131,6 +1131,30 @@ AsmTables prepare_assembly(nrg_ctx* c, const ModelSpec& m, const Basis& B, const
   return T;
 }
 
+// One matrix of a grouped GEMM launch: its index in the launch's list, rows and
+// columns.
+struct TileDim { int id, m, n; };
+
+// The matrices cut into tiles of 4 R rows x kGemmTile columns, listed by matrix in
+// (id, mn); returns R.  A tile takes R units of time (gemm_tile.cuh) and an SM one
+// tile at a time, whichever others are resident: the R with the fewest units, the
+// largest of equal ones (fewer loads).  Tangent sweep at 200 kept, 10 to 60 tiles
+// of 32 rows per launch: 50 ms with tiles of 32 rows only, 40.5 ms so.
+int cut_tiles(const std::vector<TileDim>& dims, int sms, std::vector<int>& id, std::vector<int>& mn) {
+  int best = 8;
+  int64_t least = std::numeric_limits<int64_t>::max();
+  for (int R = 8; R >= 2; R /= 2) {
+    int64_t tiles = 0;
+    for (const TileDim& d : dims) tiles += (int64_t)((d.m + 4 * R - 1) / (4 * R)) * ((d.n + kGemmTile - 1) / kGemmTile);
+    const int64_t units = (tiles + sms - 1) / sms * R;
+    if (units < least) { least = units; best = R; }
+  }
+  for (const TileDim& d : dims)
+    for (int mt = 0; mt * 4 * best < d.m; ++mt)
+      for (int nt = 0; nt * kGemmTile < d.n; ++nt) { id.push_back(d.id); mn.push_back((mt << 16) | nt); }
+  return best;
+}
+
 // UpdateMatrices for all operators: the host lists, per kept block pair
 // (i, j) allowed by CheckForMatEl, one rotation job Z_i F Z_j^T and the terms
 // of F (site factor x identity, or old operator block x identity), packed in
@@ -1142,6 +1166,7 @@ struct UpdatePlan {
   std::vector<GatherTerm> terms, terms1;
   std::vector<int> g1first, g1count, t1group, t1mn, gfirst, gcount, tjob, tmn;
   int64_t tsize = 0;
+  int rows = 8, rows1 = 8;  // of a tile, per warp
   Packer up;
   size_t o_t1 = 0, o_g1f = 0, o_g1c = 0, o_t1g = 0, o_t1m = 0, o_terms = 0, o_gf = 0, o_gc = 0, o_jobs = 0,
          o_tj = 0, o_tm = 0;
@@ -1158,7 +1183,7 @@ struct UpdatePlan {
 // kept_rows (DM-NRG shells, K = every state): per block of B its kept
 // states.  Operators other than c_d are then computed on the kept states only
 // (the next iteration reads nothing else), in the full layout.
-void plan_update(UpdatePlan& U, const ModelSpec& m, const Basis& B, const EigPlan& P, const Kept& K,
+void plan_update(UpdatePlan& U, int sms, const ModelSpec& m, const Basis& B, const EigPlan& P, const Kept& K,
                  const std::vector<OpMeta>& oldops, const std::vector<int>* opblock = nullptr,
                  const std::vector<int>* opsize = nullptr, const std::vector<int>* kept_rows = nullptr) {
   auto ob = [&](int k) { return opblock ? (*opblock)[k] : k; };
@@ -1168,6 +1193,7 @@ void plan_update(UpdatePlan& U, const ModelSpec& m, const Basis& B, const EigPla
   // The site factors depend on the two spins and the two site states only and
   // most block pairs share them: one evaluation per plan.
   const int NT = m.site.nstates;
+  std::vector<TileDim> dims, dims1;
   std::map<std::pair<double, double>, std::vector<double>> factors;  // of one operator; NaN: not yet evaluated
   for (int o = 0; o < nops; ++o) {
     OpMeta& no = U.newops[o];
@@ -1239,14 +1265,14 @@ void plan_update(UpdatePlan& U, const ModelSpec& m, const Basis& B, const EigPla
             if ((int)U.terms1.size() > first1) {
               const int gid = (int)U.g1first.size();
               U.g1first.push_back(first1); U.g1count.push_back((int)U.terms1.size() - first1);
-              for (int mt = 0; mt * kGemmTile < p.count; ++mt)
-                for (int nt = 0; nt * kGemmTile < J.kj; ++nt) { U.t1group.push_back(gid); U.t1mn.push_back((mt << 16) | nt); }
+              dims1.push_back({gid, p.count, J.kj});
             }
           }
-        for (int mt = 0; mt * kGemmTile < J.ki; ++mt)
-          for (int nt = 0; nt * kGemmTile < J.kj; ++nt) { U.tjob.push_back(jid); U.tmn.push_back((mt << 16) | nt); }
+        dims.push_back({jid, J.ki, J.kj});
       }
   }
+  U.rows = cut_tiles(dims, sms, U.tjob, U.tmn);
+  U.rows1 = cut_tiles(dims1, sms, U.t1group, U.t1mn);
   U.o_t1 = U.up.add(U.terms1); U.o_g1f = U.up.add(U.g1first); U.o_g1c = U.up.add(U.g1count);
   U.o_t1g = U.up.add(U.t1group); U.o_t1m = U.up.add(U.t1mn);
   U.o_terms = U.up.add(U.terms); U.o_gf = U.up.add(U.gfirst); U.o_gc = U.up.add(U.gcount);
@@ -1285,6 +1311,7 @@ void launch_update_plan(nrg_ctx* c, Timer& tm, UpdatePlan& U, const UpdateInputs
     if (!sub->site_terms) ua.ngroups = 0;
   }
   ua.tile_job = (const int*)(ub + U.o_tj); ua.tile_mn = (const int*)(ub + U.o_tm); ua.ntiles = (int)U.tjob.size();
+  ua.rows = U.rows; ua.rows1 = U.rows1;
   ua.terms1 = (const GatherTerm*)(ub + U.o_t1); ua.group1_first = (const int*)(ub + U.o_g1f);
   ua.group1_count = (const int*)(ub + U.o_g1c); ua.tile1_group = (const int*)(ub + U.o_t1g);
   ua.tile1_mn = (const int*)(ub + U.o_t1m); ua.ntiles1 = (int)U.t1group.size();
@@ -1298,23 +1325,22 @@ void launch_update_plan(nrg_ctx* c, Timer& tm, UpdatePlan& U, const UpdateInputs
 // Grouped FP64 GEMM jobs (gemm_jobs_kernel): one tile per CTA.
 struct GemmPlan {
   std::vector<GemmJob> jobs;
-  std::vector<int> tjob, tmn;
-  void add(const GemmJob& J) {
-    const int id = (int)jobs.size();
-    jobs.push_back(J);
-    for (int mt = 0; mt * kGemmTile < J.m; ++mt)
-      for (int nt = 0; nt * kGemmTile < J.n; ++nt) { tjob.push_back(id); tmn.push_back((mt << 16) | nt); }
-  }
+  void add(const GemmJob& J) { jobs.push_back(J); }
 };
 
 void run_gemm_plan(nrg_ctx* c, const GemmPlan& G) {
   if (G.jobs.empty()) return;
+  std::vector<TileDim> dims;
+  for (size_t k = 0; k < G.jobs.size(); ++k) dims.push_back({(int)k, G.jobs[k].m, G.jobs[k].n});
+  std::vector<int> tjob, tmn;
+  const int rows = cut_tiles(dims, c->num_sms, tjob, tmn);
   Packer pk;
-  size_t oj = pk.add(G.jobs), ot = pk.add(G.tjob), om = pk.add(G.tmn);
+  size_t oj = pk.add(G.jobs), ot = pk.add(tjob), om = pk.add(tmn);
   c->vmeta.ensure(pk.host.size() + 256);
   h2d(c, c->vmeta.p, pk.host.data(), pk.host.size());
   char* b = c->vmeta.as<char>();
-  launch_gemm_jobs((const GemmJob*)(b + oj), (const int*)(b + ot), (const int*)(b + om), (int)G.tjob.size(), c->stream);
+  launch_gemm_jobs((const GemmJob*)(b + oj), (const int*)(b + ot), (const int*)(b + om), (int)tjob.size(), rows,
+                   c->stream);
   c->launches++;
 }
 
@@ -1624,7 +1650,7 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
       Kfull.blk = B.blk;
       for (int b = 0; b < nb; ++b) Kfull.src.push_back(b);
     }
-    plan_update(U, m, B, P, fullvec ? Kfull : K, S.ops, opblock.empty() ? nullptr : &opblock, &opsize,
+    plan_update(U, c->num_sms, m, B, P, fullvec ? Kfull : K, S.ops, opblock.empty() ? nullptr : &opblock, &opsize,
                 fullvec ? &keptb : nullptr);
     std::vector<OpMeta>& newops = U.newops;
     const int nk = K.blk.nblocks();
@@ -3262,7 +3288,7 @@ void update_ops_impl(nrg_ctx* c, int model, const nrg_blocks* old_kept, const nr
     oldptr[o] = c->ops_a[o].as<double>();
   }
   UpdatePlan U;
-  plan_update(U, m, B, P, K, oldops);
+  plan_update(U, c->num_sms, m, B, P, K, oldops);
   int64_t total = 0;
   std::vector<int64_t> obase(nops);
   for (int o = 0; o < nops; ++o) {

@@ -22,25 +22,26 @@ namespace nrg {
 
 namespace {
 
+template <int RW>
 __global__ void __launch_bounds__(kGemmThreads, 6) gemm_jobs_kernel(const GemmJob* jobs, const int* tile_job,
                                                                  const int* tile_mn) {
-  __shared__ GemmSmem S;
+  __shared__ GemmSmem<RW> S;
   const GemmJob J = jobs[tile_job[blockIdx.x]];
   const int mn = tile_mn[blockIdx.x];
-  const int m0 = (mn >> 16) * kGemmTile, n0 = (mn & 0xffff) * kGemmTile;
+  const int m0 = (mn >> 16) * 4 * RW, n0 = (mn & 0xffff) * kGemmTile;
   const int rows = J.m - m0;
-  double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  double acc[RW] = {};
   auto loadB = [&](int k, int c) { return n0 + c < J.n ? J.B[(int64_t)k * J.ldb + n0 + c] : 0.0; };
   if (J.transA)
-    gemm_tile<true>(S, J.k, rows, [&](int r, int k) { return r < rows ? J.A[(int64_t)k * J.lda + m0 + r] : 0.0; },
+    gemm_tile<RW, true>(S, J.k, rows, [&](int r, int k) { return r < rows ? J.A[(int64_t)k * J.lda + m0 + r] : 0.0; },
                     loadB, acc);
   else
-    gemm_tile<false>(S, J.k, rows, [&](int r, int k) { return r < rows ? J.A[(int64_t)(m0 + r) * J.lda + k] : 0.0; },
+    gemm_tile<RW, false>(S, J.k, rows, [&](int r, int k) { return r < rows ? J.A[(int64_t)(m0 + r) * J.lda + k] : 0.0; },
                      loadB, acc);
-  const int c = n0 + (threadIdx.x & 31), r0 = m0 + 8 * (threadIdx.x >> 5);
+  const int c = n0 + (threadIdx.x & 31), r0 = m0 + RW * (threadIdx.x >> 5);
   if (c >= J.n) return;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
+  for (int i = 0; i < RW; ++i) {
     if (r0 + i >= J.m) break;
     double* o = J.C + (int64_t)(r0 + i) * J.ldc + c;
     *o = J.accum ? *o + acc[i] : acc[i];
@@ -458,8 +459,12 @@ __global__ void lehmann_fold_kernel(LehmannArgs A) {
 
 }  // namespace
 
-void launch_gemm_jobs(const GemmJob* jobs, const int* tile_job, const int* tile_mn, int ntiles, cudaStream_t s) {
-  if (ntiles > 0) gemm_jobs_kernel<<<ntiles, kGemmThreads, 0, s>>>(jobs, tile_job, tile_mn);
+void launch_gemm_jobs(const GemmJob* jobs, const int* tile_job, const int* tile_mn, int ntiles, int rows,
+                      cudaStream_t s) {
+  if (ntiles <= 0) return;
+  if (rows == 8) gemm_jobs_kernel<8><<<ntiles, kGemmThreads, 0, s>>>(jobs, tile_job, tile_mn);
+  else if (rows == 4) gemm_jobs_kernel<4><<<ntiles, kGemmThreads, 0, s>>>(jobs, tile_job, tile_mn);
+  else gemm_jobs_kernel<2><<<ntiles, kGemmThreads, 0, s>>>(jobs, tile_job, tile_mn);
 }
 
 void launch_dm_trace(const DmTraceArgs& a, int nblocks, cudaStream_t s) {

@@ -49,22 +49,23 @@ __global__ void __launch_bounds__(256) gather_kernel(UpdateArgs A) {
 }
 
 // O (ki x kj) = Z_I (ki x nI) . T (nI x kj), one tile per CTA.
+template <int RW>
 __global__ void __launch_bounds__(kGemmThreads, 6) gemm_kernel(UpdateArgs A) {
-  __shared__ GemmSmem S;
+  __shared__ GemmSmem<RW> S;
   const RotJob J = A.jobs[A.tile_job[blockIdx.x]];
   const int mn = A.tile_mn[blockIdx.x];
-  const int m0 = (mn >> 16) * kGemmTile, n0 = (mn & 0xffff) * kGemmTile;
+  const int m0 = (mn >> 16) * 4 * RW, n0 = (mn & 0xffff) * kGemmTile;
   const int rows = J.ki - m0, K = J.nI, N = J.kj;
   const double* Am = A.Z + J.z_off + (int64_t)m0 * K;
   const double* Bm = A.T + J.t_off;
-  double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  gemm_tile<false>(S, K, rows, [&](int r, int k) { return r < rows ? Am[(int64_t)r * K + k] : 0.0; },
+  double acc[RW] = {};
+  gemm_tile<RW, false>(S, K, rows, [&](int r, int k) { return r < rows ? Am[(int64_t)r * K + k] : 0.0; },
                    [&](int k, int c) { return n0 + c < N ? Bm[(int64_t)k * N + n0 + c] : 0.0; }, acc);
-  const int c = n0 + (threadIdx.x & 31), r0 = m0 + 8 * (threadIdx.x >> 5);
+  const int c = n0 + (threadIdx.x & 31), r0 = m0 + RW * (threadIdx.x >> 5);
   double* O = A.new_ops[J.op] + J.o_off;
   if (c >= N) return;
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < RW; ++i)
     if (r0 + i < J.ki) O[(int64_t)(r0 + i) * J.ldo + c] = acc[i];
 }
 
@@ -72,22 +73,23 @@ __global__ void __launch_bounds__(kGemmThreads, 6) gemm_kernel(UpdateArgs A) {
 // T[dst(a)] += sum_terms coef * sum_b M[a][b] Zt[src(b)].  The terms of one
 // group share their destination rows (one row group of one job) and are
 // summed inside the tile, so tiles of different groups never overlap.
+template <int RW>
 __global__ void __launch_bounds__(kGemmThreads, 6) imp_gemm_kernel(UpdateArgs A) {
-  __shared__ GemmSmem S;
+  __shared__ GemmSmem<RW> S;
   const int grp = A.tile1_group[blockIdx.x];
   const int t0 = A.group1_first[grp], nt = A.group1_count[grp];
   const int mn = A.tile1_mn[blockIdx.x];
   const GatherTerm G0 = A.terms1[t0];
   const RotJob J = A.jobs[G0.job];
-  const int m0 = (mn >> 16) * kGemmTile, n0 = (mn & 0xffff) * kGemmTile;
+  const int m0 = (mn >> 16) * 4 * RW, n0 = (mn & 0xffff) * kGemmTile;
   const int rows = G0.rows - m0, N = J.kj;
   const double* Zt = A.Zt + J.zt_off;
   double* T = A.T + J.t_off;
-  double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  double acc[RW] = {};
   for (int t = t0; t < t0 + nt; ++t) {
     const GatherTerm G = A.terms1[t];
     const double* Am = A.old_ops[G.op] + G.old_off + (int64_t)m0 * G.old_ld;  // rows x srows, row stride old_ld
-    gemm_tile<false>(S, G.srows, rows,
+    gemm_tile<RW, false>(S, G.srows, rows,
                      [&](int r, int k) { return r < rows ? G.coef * Am[(int64_t)r * G.old_ld + k] : 0.0; },
                      [&](int k, int c) {
                        return n0 + c < N ? Zt[(int64_t)(G.src_base + k * G.src_stride) * J.ldz + n0 + c] : 0.0;
@@ -95,10 +97,10 @@ __global__ void __launch_bounds__(kGemmThreads, 6) imp_gemm_kernel(UpdateArgs A)
                      acc);
     __syncthreads();  // the next term's first stores into S
   }
-  const int c = n0 + (threadIdx.x & 31), r0 = m0 + 8 * (threadIdx.x >> 5);
+  const int c = n0 + (threadIdx.x & 31), r0 = m0 + RW * (threadIdx.x >> 5);
   if (c >= N) return;
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < RW; ++i)
     if (r0 + i < G0.rows) T[(int64_t)(G0.dst_base + (r0 + i) * G0.dst_stride) * N + c] += acc[i];
 }
 
@@ -106,8 +108,16 @@ __global__ void __launch_bounds__(kGemmThreads, 6) imp_gemm_kernel(UpdateArgs A)
 
 void launch_update(const UpdateArgs& a, cudaStream_t s) {
   if (a.ngroups > 0) gather_kernel<<<a.ngroups, 256, 0, s>>>(a);
-  if (a.ntiles1 > 0) imp_gemm_kernel<<<a.ntiles1, kGemmThreads, 0, s>>>(a);
-  if (a.ntiles > 0) gemm_kernel<<<a.ntiles, kGemmThreads, 0, s>>>(a);
+  if (a.ntiles1 > 0) {
+    if (a.rows1 == 8) imp_gemm_kernel<8><<<a.ntiles1, kGemmThreads, 0, s>>>(a);
+    else if (a.rows1 == 4) imp_gemm_kernel<4><<<a.ntiles1, kGemmThreads, 0, s>>>(a);
+    else imp_gemm_kernel<2><<<a.ntiles1, kGemmThreads, 0, s>>>(a);
+  }
+  if (a.ntiles > 0) {
+    if (a.rows == 8) gemm_kernel<8><<<a.ntiles, kGemmThreads, 0, s>>>(a);
+    else if (a.rows == 4) gemm_kernel<4><<<a.ntiles, kGemmThreads, 0, s>>>(a);
+    else gemm_kernel<2><<<a.ntiles, kGemmThreads, 0, s>>>(a);
+  }
 }
 
 }  // namespace nrg

@@ -334,7 +334,7 @@ struct ThermoArgs {
 void launch_thermo(const ThermoArgs& a, const int* state_block, int n, double* partial, cudaStream_t s);
 
 // ---------------------------------------------------------------- update
-constexpr int kGemmTile = 32;  // tile of the grouped GEMMs (gemm_tile.cuh)
+constexpr int kGemmTile = 32;  // columns (and largest rows) of a tile of the grouped GEMMs (gemm_tile.cuh)
 struct GatherTerm {       // T[dst rows] += coef * M . Zt[src rows]
   int job;                // rotation job
   int dst_base, dst_stride, rows;   // rows of T (local to the job's T)
@@ -367,7 +367,7 @@ struct UpdateArgs {
   double* const* new_ops;
   const int* tile_job;    // GEMM tiles: job
   const int* tile_mn;     // GEMM tiles: (mtile << 16) | ntile
-  int ntiles;
+  int ntiles, rows;     // tiles of 4 rows x kGemmTile elements
   // impurity-operator terms (mode 1) as GEMM tiles; the terms of one group
   // share their destination rows and are summed inside one tile
   const GatherTerm* terms1;
@@ -375,7 +375,7 @@ struct UpdateArgs {
   const int* group1_count;
   const int* tile1_group;
   const int* tile1_mn;
-  int ntiles1;
+  int ntiles1, rows1;
 };
 void launch_update(const UpdateArgs& a, cudaStream_t s);
 
@@ -453,9 +453,10 @@ struct GemmJob {          // C (m x n) = op(A) (m x k) . B (k x n), row-major, F
   int ldc;
   int accum;              // 1: C += op(A) . B (after the launches that write C before)
 };
-// One kGemmTile-square tile of C per CTA: tile t belongs to job tile_job[t] at
+// One tile of C (4 rows x kGemmTile elements; rows = 8, 4 or 2) per CTA: tile t belongs to job tile_job[t] at
 // (tile_mn[t] >> 16, tile_mn[t] & 0xffff).
-void launch_gemm_jobs(const GemmJob* jobs, const int* tile_job, const int* tile_mn, int ntiles, cudaStream_t s);
+void launch_gemm_jobs(const GemmJob* jobs, const int* tile_job, const int* tile_mn, int ntiles, int rows,
+                      cudaStream_t s);
 
 struct DmTraceTerm {      // rho_N(i,j) += cg * rot[(base + i*stride) * nb + base + j*stride]
   int64_t rot_off;        // the child block of the rotated rho_{N+1} (dense nb x nb)
