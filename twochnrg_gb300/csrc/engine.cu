@@ -2959,31 +2959,33 @@ void diag_blocks_impl(nrg_ctx* c, int nb, const int* sizes, const double* packed
   Timer tm(c);
   EigPlan P;
   plan_blocks(P, bs);
-  std::vector<double> Hh((size_t)P.hsize);
-  size_t pos = 0;
-  for (int b = 0; b < nb; ++b) {
-    const int n = bs[b];
-    double* h = Hh.data() + P.hoff[b];
-    for (int i = 0; i < n; ++i)
-      for (int j = i; j < n; ++j) { const double v = packed[pos++]; h[(size_t)i * n + j] = v; h[(size_t)j * n + i] = v; }
-  }
+  std::vector<int64_t> poff(nb);
+  int64_t npacked = 0;
+  for (int b = 0; b < nb; ++b) { poff[b] = npacked; npacked += (int64_t)bs[b] * (bs[b] + 1) / 2; }
   std::vector<int> order(nb), state_block(P.nstates);
   for (int b = 0; b < nb; ++b) order[b] = b;
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return bs[x] > bs[y]; });
   for (int b = 0; b < nb; ++b) for (int i = 0; i < bs[b]; ++i) state_block[P.soff[b] + i] = b;
   Packer pk;
   size_t o_bsize = pk.add(P.bsize), o_soff = pk.add(P.soff), o_hoff = pk.add(P.hoff), o_order = pk.add(order),
-         o_sb = pk.add(state_block);
+         o_sb = pk.add(state_block), o_poff = pk.add(poff);
   c->meta.ensure(pk.host.size() + 256);
   c->H.ensure(sizeof(double) * (size_t)P.hsize);
+  c->T.ensure(sizeof(double) * (size_t)npacked);
   c->d.ensure(sizeof(double) * P.nstates); c->e.ensure(sizeof(double) * P.nstates);
   c->tau.ensure(sizeof(double) * P.nstates); c->ev.ensure(sizeof(double) * P.nstates);
   c->red.ensure(sizeof(int) * 8);
   c->flag.ensure(sizeof(int) * 4);
   CU(cudaMemsetAsync(c->flag.p, 0, sizeof(int), c->stream));
   h2d(c, c->meta.p, pk.host.data(), pk.host.size());
-  h2d(c, c->H.p, Hh.data(), sizeof(double) * (size_t)P.hsize);
+  h2d(c, c->T.p, packed, sizeof(double) * (size_t)npacked);
   char* mb = c->meta.as<char>();
+  UnpackArgs ua{};
+  ua.packed = c->T.as<double>(); ua.poff = (const int64_t*)(mb + o_poff); ua.hoff = (const int64_t*)(mb + o_hoff);
+  ua.bsize = (const int*)(mb + o_bsize); ua.soff = (const int*)(mb + o_soff);
+  ua.state_block = (const int*)(mb + o_sb); ua.H = c->H.as<double>();
+  launch_unpack(ua, P.nstates, c->stream);
+  c->launches++;
   run_tridiag_and_bisect(c, tm, P, order, (const int*)(mb + o_order), (const int*)(mb + o_bsize),
                          (const int64_t*)(mb + o_hoff), (const int*)(mb + o_soff), (const int*)(mb + o_sb));
   std::vector<double> ev(P.nstates);

@@ -113,7 +113,27 @@ __global__ void __launch_bounds__(256) assemble_kernel(AssembleArgs A, const int
   }
 }
 
+// Symmetric blocks from their packed upper triangles (row by row), one CTA per
+// row: the row's part right of the diagonal and, mirrored, the column's below it.
+// Half the bytes over the host link and no full matrix built on the host; 1901
+// states take 2.2 ms of a host core and as much again for the zeroed copy, the
+// kernel 16 us.
+__global__ void __launch_bounds__(256) unpack_kernel(UnpackArgs A) {
+  const int s = blockIdx.x, b = A.state_block[s], i = s - A.soff[b], n = A.bsize[b];
+  const double* src = A.packed + A.poff[b] + (int64_t)i * n - (int64_t)i * (i - 1) / 2 - i;  // element j at src[j]
+  double* H = A.H + A.hoff[b];
+  for (int j = i + threadIdx.x; j < n; j += blockDim.x) {
+    const double v = src[j];
+    H[(int64_t)i * n + j] = v;
+    H[(int64_t)j * n + i] = v;
+  }
+}
+
 }  // namespace
+
+void launch_unpack(const UnpackArgs& a, int nstates, cudaStream_t s) {
+  if (nstates > 0) unpack_kernel<<<nstates, 256, 0, s>>>(a);
+}
 
 void launch_assemble(const AssembleArgs& a, int64_t total_rows, const int* row_block, const int* row_index,
                      cudaStream_t s) {

@@ -180,6 +180,17 @@ struct AssembleArgs {
   const int* hc_switch;      // [ntypes^2]; model 5: [2 * ntypes^2], spin up first
   double delta;
 };
+// Blocks from packed upper triangles; block b's at packed + poff[b].
+struct UnpackArgs {
+  const double* packed;
+  const int64_t* poff;
+  const int64_t* hoff;
+  const int* bsize;
+  const int* soff;
+  const int* state_block;
+  double* H;
+};
+void launch_unpack(const UnpackArgs& a, int nstates, cudaStream_t s);
 void launch_assemble(const AssembleArgs& a, int64_t total_rows, const int* row_block,
                      const int* row_index, cudaStream_t s);
 
