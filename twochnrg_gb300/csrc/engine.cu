@@ -1138,15 +1138,15 @@ struct TileDim { int id, m, n; };
 // The matrices cut into tiles of 4 R rows x kGemmTile columns, listed by matrix in
 // (id, mn); returns R.  A tile takes R units of time (gemm_tile.cuh) and an SM one
 // tile at a time, whichever others are resident: the R with the fewest units, the
-// largest of equal ones (fewer loads).  Tangent sweep at 200 kept, 10 to 60 tiles
+// largest of equal ones (fewer loads).  The list is run `times` times in one launch.  Tangent sweep at 200 kept, 10 to 60 tiles
 // of 32 rows per launch: 50 ms with tiles of 32 rows only, 40.5 ms so.
-int cut_tiles(const std::vector<TileDim>& dims, int sms, std::vector<int>& id, std::vector<int>& mn) {
+int cut_tiles(const std::vector<TileDim>& dims, int sms, int times, std::vector<int>& id, std::vector<int>& mn) {
   int best = 8;
   int64_t least = std::numeric_limits<int64_t>::max();
   for (int R = 8; R >= 2; R /= 2) {
     int64_t tiles = 0;
     for (const TileDim& d : dims) tiles += (int64_t)((d.m + 4 * R - 1) / (4 * R)) * ((d.n + kGemmTile - 1) / kGemmTile);
-    const int64_t units = (tiles + sms - 1) / sms * R;
+    const int64_t units = (tiles * times + sms - 1) / sms * R;
     if (units < least) { least = units; best = R; }
   }
   for (const TileDim& d : dims)
@@ -1159,7 +1159,8 @@ int cut_tiles(const std::vector<TileDim>& dims, int sms, std::vector<int>& id, s
 // (i, j) allowed by CheckForMatEl, one rotation job Z_i F Z_j^T and the terms
 // of F (site factor x identity, or old operator block x identity), packed in
 // `up`.  The caller adds the operator pointer tables (o_old, o_new) and any
-// tables of its own to `up` before launch_update_plan.
+// tables of its own to `up` before launch_update_plan.  ndir: the directions of a
+// tangent pass, whose launches are the larger ones then.
 struct UpdatePlan {
   std::vector<OpMeta> newops;
   std::vector<RotJob> jobs;
@@ -1183,7 +1184,7 @@ struct UpdatePlan {
 // kept_rows (DM-NRG shells, K = every state): per block of B its kept
 // states.  Operators other than c_d are then computed on the kept states only
 // (the next iteration reads nothing else), in the full layout.
-void plan_update(UpdatePlan& U, int sms, const ModelSpec& m, const Basis& B, const EigPlan& P, const Kept& K,
+void plan_update(UpdatePlan& U, int sms, int ndir, const ModelSpec& m, const Basis& B, const EigPlan& P, const Kept& K,
                  const std::vector<OpMeta>& oldops, const std::vector<int>* opblock = nullptr,
                  const std::vector<int>* opsize = nullptr, const std::vector<int>* kept_rows = nullptr) {
   auto ob = [&](int k) { return opblock ? (*opblock)[k] : k; };
@@ -1271,54 +1272,68 @@ void plan_update(UpdatePlan& U, int sms, const ModelSpec& m, const Basis& B, con
         dims.push_back({jid, J.ki, J.kj});
       }
   }
-  U.rows = cut_tiles(dims, sms, U.tjob, U.tmn);
-  U.rows1 = cut_tiles(dims1, sms, U.t1group, U.t1mn);
+  U.rows = cut_tiles(dims, sms, ndir, U.tjob, U.tmn);
+  U.rows1 = cut_tiles(dims1, sms, ndir, U.t1group, U.t1mn);
   U.o_t1 = U.up.add(U.terms1); U.o_g1f = U.up.add(U.g1first); U.o_g1c = U.up.add(U.g1count);
   U.o_t1g = U.up.add(U.t1group); U.o_t1m = U.up.add(U.t1mn);
   U.o_terms = U.up.add(U.terms); U.o_gf = U.up.add(U.gfirst); U.o_gc = U.up.add(U.gcount);
   U.o_jobs = U.up.add(U.jobs); U.o_tj = U.up.add(U.tjob); U.o_tm = U.up.add(U.tmn);
 }
 
-// Substitutions for a run of an update plan with other inputs (the tangent
-// pass): eigenvector rows Z and columns Zt, device tables of old and new
-// operator pointers, and whether the site-operator (identity-on-old) terms
-// take part.
-struct UpdateInputs {
-  const double* Z = nullptr;
-  const double* Zt = nullptr;
-  const double* const* old_tab = nullptr;
-  double* const* new_tab = nullptr;
-  bool site_terms = true;
-};
-
-void launch_update_plan(nrg_ctx* c, Timer& tm, UpdatePlan& U, const UpdateInputs* sub = nullptr) {
-  cudaEvent_t tu = tm.start();
-  const size_t tbytes = sizeof(double) * std::max<int64_t>(U.tsize, 1);
-  if (!sub) {
-    c->T.ensure(tbytes + U.up.host.size() + 512);
-    U.ub = c->T.as<char>() + ((tbytes + 255) & ~size_t(255));
-    h2d(c, U.ub, U.up.host.data(), U.up.host.size());
-  }
-  CU(cudaMemsetAsync(c->T.p, 0, tbytes, c->stream));
+UpdateArgs update_args(nrg_ctx* c, const UpdatePlan& U) {
   char* ub = U.ub;
   UpdateArgs ua{};
   ua.terms = (const GatherTerm*)(ub + U.o_terms); ua.group_first = (const int*)(ub + U.o_gf);
   ua.group_count = (const int*)(ub + U.o_gc); ua.ngroups = (int)U.gfirst.size(); ua.jobs = (const RotJob*)(ub + U.o_jobs);
   ua.Z = c->Z.as<double>(); ua.Zt = c->Zt.as<double>(); ua.T = c->T.as<double>();
   ua.old_ops = (const double* const*)(ub + U.o_old); ua.new_ops = (double* const*)(ub + U.o_new);
-  if (sub) {
-    ua.Z = sub->Z; ua.Zt = sub->Zt; ua.old_ops = sub->old_tab; ua.new_ops = sub->new_tab;
-    if (!sub->site_terms) ua.ngroups = 0;
-  }
   ua.tile_job = (const int*)(ub + U.o_tj); ua.tile_mn = (const int*)(ub + U.o_tm); ua.ntiles = (int)U.tjob.size();
   ua.rows = U.rows; ua.rows1 = U.rows1;
   ua.terms1 = (const GatherTerm*)(ub + U.o_t1); ua.group1_first = (const int*)(ub + U.o_g1f);
   ua.group1_count = (const int*)(ub + U.o_g1c); ua.tile1_group = (const int*)(ub + U.o_t1g);
   ua.tile1_mn = (const int*)(ub + U.o_t1m); ua.ntiles1 = (int)U.t1group.size();
+  return ua;
+}
+
+void launch_update_plan(nrg_ctx* c, Timer& tm, UpdatePlan& U) {
+  cudaEvent_t tu = tm.start();
+  const size_t tbytes = sizeof(double) * std::max<int64_t>(U.tsize, 1);
+  c->T.ensure(tbytes + U.up.host.size() + 512);
+  U.ub = c->T.as<char>() + ((tbytes + 255) & ~size_t(255));
+  h2d(c, U.ub, U.up.host.data(), U.up.host.size());
+  CU(cudaMemsetAsync(c->T.p, 0, tbytes, c->stream));
+  const UpdateArgs ua = update_args(c, U);
   launch_update(ua, c->stream);
   if (ua.ntiles1 > 0) c->launches++;
   c->launches += 2;
   for (const RotJob& J : U.jobs) c->timing.update_flops += 2.0 * J.ki * (double)J.nI * J.kj;
+  tm.stop(tu, &c->timing.update_ms);
+}
+
+// The tangents of the plan's operators in all directions, after
+// launch_update_plan (whose T it reads).
+struct UpdateTangents {
+  const double* dZ;
+  const double* dZt;
+  int64_t z_stride;
+  DevBuf* dT;
+  const double* const* old_tab;  // 16 pointers per direction
+  double* const* new_tab;
+};
+
+void launch_update_tangents(nrg_ctx* c, Timer& tm, UpdatePlan& U, const UpdateTangents& t) {
+  cudaEvent_t tu = tm.start();
+  const int64_t ts = std::max<int64_t>(U.tsize, 1);
+  t.dT->ensure(sizeof(double) * kTanDirs * ts);
+  CU(cudaMemsetAsync(t.dT->p, 0, sizeof(double) * kTanDirs * ts, c->stream));
+  UpdateArgs ua = update_args(c, U);
+  ua.ndir = kTanDirs;
+  ua.dZ = t.dZ; ua.dZt = t.dZt; ua.z_stride = t.z_stride; ua.dT = t.dT->as<double>(); ua.t_stride = ts;
+  ua.dold_ops = t.old_tab; ua.dnew_ops = t.new_tab;
+  launch_update(ua, c->stream);
+  if (ua.ntiles1 > 0) c->launches++;
+  c->launches += 2;
+  for (const RotJob& J : U.jobs) c->timing.update_flops += 2.0 * kTanDirs * 2.0 * J.ki * (double)J.nI * J.kj;
   tm.stop(tu, &c->timing.update_ms);
 }
 
@@ -1333,7 +1348,7 @@ void run_gemm_plan(nrg_ctx* c, const GemmPlan& G) {
   std::vector<TileDim> dims;
   for (size_t k = 0; k < G.jobs.size(); ++k) dims.push_back({(int)k, G.jobs[k].m, G.jobs[k].n});
   std::vector<int> tjob, tmn;
-  const int rows = cut_tiles(dims, c->num_sms, tjob, tmn);
+  const int rows = cut_tiles(dims, c->num_sms, 1, tjob, tmn);
   Packer pk;
   size_t oj = pk.add(G.jobs), ot = pk.add(tjob), om = pk.add(tmn);
   c->vmeta.ensure(pk.host.size() + 256);
@@ -1350,10 +1365,12 @@ void run_gemm_plan(nrg_ctx* c, const GemmPlan& G) {
 // (ping-pong buffers like the primal operators), the scratch of the
 // eigen-derivatives, and the per-iteration results.
 struct TangentState {
-  static constexpr int NP = 4;
+  static constexpr int NP = kTanDirs;
   double params[NP] = {0, 0, 0, 0};     // eps_d, U, Gamma, B of the sweep
-  DevBuf dEk[NP][2], dops[NP][2][6];
-  DevBuf deold, dH, T1, dHt, C, dZ, dZt, dlam, dEall, tmp[3][6], gscaled[6], tabs, part, out;
+  // every buffer holds the parameters' arrays one after the other
+  DevBuf dEk[2], dops[2][6];
+  int64_t nEk[2] = {0, 0}, nop[2][6] = {};  // length of one parameter's array
+  DevBuf deold, dH, T1, dHt, C, dZ, dZt, dT, dlam, dEall, gscaled[6], tabs, part, out;
   // per iteration n and parameter k (index n * NP + k): tangents of the
   // thermodynamic values (the 16 of nrg_iteration.thermo), of the operator
   // averages, and of the raw lowest level (lambda_min, before SetE0zero)
@@ -1507,16 +1524,20 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
                               make_start(m, lambda, 0.0, 0.0, 1.0)};
     tan->params[0] = cfg->ed; tan->params[1] = cfg->U; tan->params[2] = cfg->gamma1; tan->params[3] = cfg->gamma2_or_B;
     tan->dthermo.clear(); tan->dopavg.clear(); tan->dlmin.clear();
-    for (int p = 0; p < TangentState::NP; ++p) {
-      std::vector<double> de(st.en.size(), 0.0);
+    const int NP = TangentState::NP;
+    const size_t ne = st.en.size();
+    std::vector<double> de(NP * ne, 0.0);
+    for (int p = 0; p < NP; ++p)
       if (p != 2)
-        for (size_t k = 0; k < de.size(); ++k) de[k] = sd[p == 3 ? 2 : p].en[k] - s0.en[k];
-      tan->dEk[p][0].ensure(sizeof(double) * std::max<size_t>(de.size(), 1));
-      h2d(c, tan->dEk[p][0].p, de.data(), sizeof(double) * de.size());
-      for (int o = 0; o < nops; ++o) {
-        tan->dops[p][0][o].ensure(sizeof(double) * std::max<int64_t>(S.ops[o].size, 1));
-        CU(cudaMemsetAsync(tan->dops[p][0][o].p, 0, sizeof(double) * std::max<int64_t>(S.ops[o].size, 1), c->stream));
-      }
+        for (size_t k = 0; k < ne; ++k) de[p * ne + k] = sd[p == 3 ? 2 : p].en[k] - s0.en[k];
+    tan->nEk[0] = (int64_t)ne;
+    tan->dEk[0].ensure(sizeof(double) * std::max<size_t>(de.size(), 1));
+    h2d(c, tan->dEk[0].p, de.data(), sizeof(double) * de.size());
+    for (int o = 0; o < nops; ++o) {
+      const int64_t sz = std::max<int64_t>(S.ops[o].size, 1);
+      tan->nop[0][o] = sz;
+      tan->dops[0][o].ensure(sizeof(double) * NP * sz);
+      CU(cudaMemsetAsync(tan->dops[0][o].p, 0, sizeof(double) * NP * sz, c->stream));
     }
   }
   int tcur = 0;  // which tangent ping-pong buffer holds the current tangents
@@ -1650,7 +1671,7 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
       Kfull.blk = B.blk;
       for (int b = 0; b < nb; ++b) Kfull.src.push_back(b);
     }
-    plan_update(U, c->num_sms, m, B, P, fullvec ? Kfull : K, S.ops, opblock.empty() ? nullptr : &opblock, &opsize,
+    plan_update(U, c->num_sms, tan ? kTanDirs : 1, m, B, P, fullvec ? Kfull : K, S.ops, opblock.empty() ? nullptr : &opblock, &opsize,
                 fullvec ? &keptb : nullptr);
     std::vector<OpMeta>& newops = U.newops;
     const int nk = K.blk.nblocks();
@@ -1730,19 +1751,24 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
       int gs = 0;
       for (int g = 1; g < P.nstates; ++g) if (R.en[g] < R.en[gs]) gs = g;
       const int nkept = (int)kept_state.size();
-      TS.deold.ensure(sizeof(double) * std::max(P.nstates, 1));
-      for (DevBuf* b : {&TS.dH, &TS.T1, &TS.dHt}) b->ensure(sizeof(double) * std::max<int64_t>(P.hsize, 1));
-      TS.C.ensure(sizeof(double) * std::max<int64_t>(csz, 1));
-      TS.dZ.ensure(sizeof(double) * std::max<int64_t>(P.ysize, 1));
-      TS.dZt.ensure(sizeof(double) * std::max<int64_t>(P.ysize, 1));
-      TS.dlam.ensure(sizeof(double) * std::max(P.nstates, 1));
-      TS.dEall.ensure(sizeof(double) * std::max(P.nstates, 1));
-      for (int r = 0; r < 3; ++r)
-        for (int o = 0; o < nops; ++o) TS.tmp[r][o].ensure(sizeof(double) * std::max<int64_t>(newops[o].size, 1));
-      for (int p = 0; p < NP; ++p) {
-        TS.dEk[p][1 - tcur].ensure(sizeof(double) * std::max(nkept, 1));
-        for (int o = 0; o < nops; ++o)
-          TS.dops[p][1 - tcur][o].ensure(sizeof(double) * std::max<int64_t>(newops[o].size, 1));
+      const int64_t ns = P.nstates, hs = std::max<int64_t>(P.hsize, 1), ys = std::max<int64_t>(P.ysize, 1),
+                    cs = std::max<int64_t>(csz, 1);
+      const int tnext = 1 - tcur;
+      TS.deold.ensure(sizeof(double) * NP * std::max<int64_t>(ns, 1));
+      for (DevBuf* b : {&TS.dH, &TS.T1, &TS.dHt}) b->ensure(sizeof(double) * NP * hs);
+      TS.C.ensure(sizeof(double) * NP * cs);
+      TS.dZ.ensure(sizeof(double) * NP * ys);
+      TS.dZt.ensure(sizeof(double) * NP * ys);
+      TS.dlam.ensure(sizeof(double) * NP * std::max<int64_t>(ns, 1));
+      TS.dEall.ensure(sizeof(double) * NP * std::max<int64_t>(ns, 1));
+      TS.nEk[tnext] = nkept;
+      TS.dEk[tnext].ensure(sizeof(double) * NP * std::max(nkept, 1));
+      for (int o = 0; o < nops; ++o) {
+        const int64_t sz = std::max<int64_t>(newops[o].size, 1);
+        TS.nop[tnext][o] = sz;
+        TS.dops[tnext][o].ensure(sizeof(double) * NP * sz);
+        // only the kept part of a full-layout operator is computed
+        CU(cudaMemsetAsync(TS.dops[tnext][o].p, 0, sizeof(double) * NP * sz, c->stream));
       }
       // iteration 0, Gamma: chi_{-1} is proportional to sqrt(Gamma), so the
       // coupling's tangent is the primal coupling over 2 Gamma
@@ -1753,20 +1779,21 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
           launch_tan_scale(S.opbuf(S.cur, o)->as<double>(), 0.5 / cfg->gamma1, S.ops[o].size,
                            TS.gscaled[o].as<double>(), c->stream);
         }
-      // pointer tables: per parameter the tangent old operators (8) and new
-      // ones (8), then the three rotation outputs (8 each), the Gamma-scaled
-      // couplings (8), and per parameter the averaged operators' tangents (8)
+      // pointer tables: per parameter the tangents of the old operators (8) and
+      // of the new ones (8); the old ones as they enter H_N (the Gamma-scaled
+      // couplings in iteration 0); the averaged operators' (8 per parameter each)
       std::vector<const double*> ptrs;
+      auto op_tan = [&](int which, int o, int p) { return TS.dops[which][o].as<double>() + p * TS.nop[which][o]; };
       for (int p = 0; p < NP; ++p) {
-        for (int o = 0; o < 8; ++o) ptrs.push_back(o < nops ? TS.dops[p][tcur][o].as<double>() : nullptr);
-        for (int o = 0; o < 8; ++o) ptrs.push_back(o < nops ? TS.dops[p][1 - tcur][o].as<double>() : nullptr);
+        for (int o = 0; o < 8; ++o) ptrs.push_back(o < nops ? op_tan(tcur, o, p) : nullptr);
+        for (int o = 0; o < 8; ++o) ptrs.push_back(o < nops ? op_tan(tnext, o, p) : nullptr);
       }
-      for (int r = 0; r < 3; ++r)
-        for (int o = 0; o < 8; ++o) ptrs.push_back(o < nops ? TS.tmp[r][o].as<double>() : nullptr);
-      for (int o = 0; o < 8; ++o) ptrs.push_back(gamma_term && o < nops_h ? TS.gscaled[o].as<double>() : nullptr);
       for (int p = 0; p < NP; ++p)
-        for (int k = 0; k < 8; ++k)
-          ptrs.push_back(k < (int)avg_ops.size() ? TS.dops[p][1 - tcur][avg_ops[k]].as<double>() : nullptr);
+        for (int o = 0; o < 8; ++o)
+          ptrs.push_back(gamma_term && p == 2 ? (o < nops_h ? TS.gscaled[o].as<double>() : nullptr)
+                                              : (o < nops ? op_tan(tcur, o, p) : nullptr));
+      for (int p = 0; p < NP; ++p)
+        for (int k = 0; k < 8; ++k) ptrs.push_back(k < (int)avg_ops.size() ? op_tan(tnext, avg_ops[k], p) : nullptr);
       Packer tp;
       const size_t o_ptr = tp.add(ptrs), o_kst = tp.add(kept_state), o_coff = tp.add(coff), o_nkeep = tp.add(ccols),
                    o_stcf = tp.add(B.stcf);
@@ -1774,87 +1801,77 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
       h2d(c, TS.tabs.p, tp.host.data(), tp.host.size());
       char* tb = TS.tabs.as<char>();
       const double* const* dptr = (const double* const*)(tb + o_ptr);
-      auto tab_old = [&](int p) { return dptr + 16 * p; };
-      auto tab_tmp = [&](int r) { return dptr + 16 * NP + 8 * r; };
-      const double* const* tab_gamma = dptr + 16 * NP + 24;
-      auto tab_avg = [&](int p) { return dptr + 16 * NP + 32 + 8 * p; };
-      // the eigen-derivative GEMMs of every block (the same for all parameters)
+      const double* const* tab_hn = dptr + 16 * NP;
+      const double* const* tab_avg = dptr + 24 * NP;
+      // the eigen-derivative GEMMs of every block and parameter
       GemmPlan G1, G2, G3, G4;
-      for (int b = 0; b < nb; ++b) {
-        const int n = P.bsize[b], kb = ccols[b];
-        const int64_t h = P.hoff[b], y = P.yoff[b];
-        double* Zb = c->Z.as<double>() + y;
-        double* Ztb = c->Zt.as<double>() + y;
-        G1.add(GemmJob{n, n, n, 0, TS.dH.as<double>() + h, n, Ztb, n, TS.T1.as<double>() + h, n});
-        G2.add(GemmJob{n, n, n, 0, Zb, n, TS.T1.as<double>() + h, n, TS.dHt.as<double>() + h, n});
-        if (kb == 0) continue;
-        G3.add(GemmJob{n, kb, n, 0, Ztb, n, TS.C.as<double>() + coff[b], kb, TS.dZt.as<double>() + y, n});
-        G4.add(GemmJob{kb, n, n, 1, TS.C.as<double>() + coff[b], kb, Zb, n, TS.dZ.as<double>() + y, n});
-      }
-      TS.part.ensure(sizeof(double) * tan_partial_doubles());
-      TS.out.ensure(sizeof(double) * TanSumArgs::kMaxOut * NP + 64);
-      std::vector<double> sums((size_t)TanSumArgs::kMaxOut * NP), dl(NP);
-      if (dm) {
-        shp->ntan = NP;
-        shp->den.assign((size_t)NP * P.nstates, 0.0);
-      }
-      for (int p = 0; p < NP; ++p) {
-        // dH_N: the assembly on the tangents of the old energies and operators
-        launch_tan_gather(TS.dEk[p][tcur].as<double>(), (const int*)(tb + o_stcf), P.nstates, TS.deold.as<double>(),
-                          c->stream);
-        AssembleArgs a2 = aa;
-        a2.H = TS.dH.as<double>(); a2.st_eold = TS.deold.as<double>(); a2.eN = 0.0;
-        a2.ops = (gamma_term && p == 2) ? tab_gamma : tab_old(p);
-        launch_assemble(a2, P.nstates, (const int*)(mb + o_sb), (const int*)(mb + AT.o_ri), c->stream);
-        run_gemm_plan(c, G1);
-        run_gemm_plan(c, G2);
-        TanEigArgs te{};
-        te.bsize = aa.bsize; te.soff = aa.bstate; te.hoff = aa.hoff; te.dHt = TS.dHt.as<double>();
-        te.ev = c->ev.as<double>(); te.nkeep = (const int*)(tb + o_nkeep); te.coff = (const int64_t*)(tb + o_coff);
-        te.C = TS.C.as<double>(); te.dlam = TS.dlam.as<double>(); te.degen_tol = 1e-10;
-        launch_tan_eig(te, nb, c->stream);
-        run_gemm_plan(c, G3);
-        run_gemm_plan(c, G4);
-        launch_tan_shift(TS.dlam.as<double>(), P.nstates, gs, TS.dEall.as<double>(), (const int*)(tb + o_kst), nkept,
-                         TS.dEk[p][1 - tcur].as<double>(), c->stream);
-        if (dm) {  // the shell's tangents: every eigenvector's and every energy's
-          shp->dZ[p].ensure(sizeof(double) * std::max<int64_t>(P.ysize, 1));
-          CU(cudaMemcpyAsync(shp->dZ[p].p, TS.dZ.p, sizeof(double) * P.ysize, cudaMemcpyDeviceToDevice, c->stream));
-          d2h(c, shp->den.data() + (size_t)p * P.nstates, TS.dEall.p, sizeof(double) * P.nstates);
+      for (int p = 0; p < NP; ++p)
+        for (int b = 0; b < nb; ++b) {
+          const int n = P.bsize[b], kb = ccols[b];
+          const int64_t h = p * hs + P.hoff[b], y = p * ys + P.yoff[b], cf = p * cs + coff[b];
+          double* Zb = c->Z.as<double>() + P.yoff[b];
+          double* Ztb = c->Zt.as<double>() + P.yoff[b];
+          G1.add(GemmJob{n, n, n, 0, TS.dH.as<double>() + h, n, Ztb, n, TS.T1.as<double>() + h, n});
+          G2.add(GemmJob{n, n, n, 0, Zb, n, TS.T1.as<double>() + h, n, TS.dHt.as<double>() + h, n});
+          if (kb == 0) continue;
+          G3.add(GemmJob{n, kb, n, 0, Ztb, n, TS.C.as<double>() + cf, kb, TS.dZt.as<double>() + y, n});
+          G4.add(GemmJob{kb, n, n, 1, TS.C.as<double>() + cf, kb, Zb, n, TS.dZ.as<double>() + y, n});
         }
-        // dO_new = dZ_I F Z_J^T + Z_I F dZ_J^T + Z_I dF Z_J^T
-        for (int r = 0; r < 3; ++r)
-          for (int o = 0; o < nops; ++o)
-            CU(cudaMemsetAsync(TS.tmp[r][o].p, 0, sizeof(double) * newops[o].size, c->stream));
-        const double* const* old_primal = (const double* const*)(ub + U.o_old);
-        UpdateInputs u1{TS.dZ.as<double>(), c->Zt.as<double>(), old_primal, (double* const*)tab_tmp(0), true};
-        UpdateInputs u2{c->Z.as<double>(), TS.dZt.as<double>(), old_primal, (double* const*)tab_tmp(1), true};
-        UpdateInputs u3{c->Z.as<double>(), c->Zt.as<double>(), tab_old(p), (double* const*)tab_tmp(2), false};
-        launch_update_plan(c, tm, U, &u1);
-        launch_update_plan(c, tm, U, &u2);
-        launch_update_plan(c, tm, U, &u3);
-        for (int o = 0; o < nops; ++o)
-          launch_tan_axpy3(TS.tmp[0][o].as<double>(), TS.tmp[1][o].as<double>(), TS.tmp[2][o].as<double>(), 1.0,
-                           newops[o].size, TS.dops[p][1 - tcur][o].as<double>(), c->stream);
-        if (dm) {
-          const int64_t ncd = newops[nops_h].size;
-          shp->dcd[p].ensure(sizeof(double) * std::max<int64_t>(ncd, 1));
-          CU(cudaMemcpyAsync(shp->dcd[p].p, TS.dops[p][1 - tcur][nops_h].p, sizeof(double) * ncd,
+      TS.part.ensure(sizeof(double) * tan_partial_doubles());
+      TS.out.ensure(sizeof(double) * (TanSumArgs::kMaxOut + 1) * NP);
+      std::vector<double> sums((size_t)(TanSumArgs::kMaxOut + 1) * NP);  // the last NP: d lambda of the ground state
+      double* const dl = sums.data() + (size_t)TanSumArgs::kMaxOut * NP;
+      // dH_N: the assembly on the tangents of the old energies and operators
+      launch_tan_gather(TS.dEk[tcur].as<double>(), (int)TS.nEk[tcur], (const int*)(tb + o_stcf), P.nstates,
+                        TS.deold.as<double>(), c->stream);
+      AssembleArgs a2 = aa;
+      a2.H = TS.dH.as<double>(); a2.st_eold = TS.deold.as<double>(); a2.eN = 0.0; a2.ops = tab_hn;
+      a2.h_stride = hs; a2.e_stride = ns;
+      launch_assemble(a2, P.nstates, (const int*)(mb + o_sb), (const int*)(mb + AT.o_ri), c->stream, NP);
+      run_gemm_plan(c, G1);
+      run_gemm_plan(c, G2);
+      TanEigArgs te{};
+      te.bsize = aa.bsize; te.soff = aa.bstate; te.hoff = aa.hoff; te.dHt = TS.dHt.as<double>();
+      te.ev = c->ev.as<double>(); te.nkeep = (const int*)(tb + o_nkeep); te.coff = (const int64_t*)(tb + o_coff);
+      te.C = TS.C.as<double>(); te.dlam = TS.dlam.as<double>(); te.degen_tol = 1e-10;
+      te.h_stride = hs; te.c_stride = cs; te.nstates = P.nstates;
+      launch_tan_eig(te, nb, c->stream);
+      run_gemm_plan(c, G3);
+      run_gemm_plan(c, G4);
+      launch_tan_shift(TS.dlam.as<double>(), P.nstates, gs, TS.dEall.as<double>(), (const int*)(tb + o_kst), nkept,
+                       TS.dEk[tnext].as<double>(), TS.out.as<double>() + TanSumArgs::kMaxOut * NP, c->stream);
+      if (dm) {  // the shell's tangents: every eigenvector's and every energy's
+        shp->ntan = NP;
+        shp->den.assign((size_t)(NP * ns), 0.0);
+        for (int p = 0; p < NP; ++p) {
+          shp->dZ[p].ensure(sizeof(double) * ys);
+          CU(cudaMemcpyAsync(shp->dZ[p].p, TS.dZ.as<double>() + p * ys, sizeof(double) * P.ysize,
                              cudaMemcpyDeviceToDevice, c->stream));
         }
-        // weighted sums of the thermodynamics and operator-average tangents
-        TanSumArgs ts{};
-        ts.nstates = P.nstates; ts.state_block = (const int*)(mb + o_sb); ts.bq = (const double*)(mb + o_bq);
-        ts.en = c->en.as<double>(); ts.dE = TS.dEall.as<double>(); ts.totalS = m.totalS ? 1 : 0;
-        for (int t = 0; t < 4; ++t) ts.beta[t] = betas[t];
-        ts.nkept = nkept; ts.nkblocks = nk; ts.kstate_block = (const int*)(ub + o_ksb); ts.koff = (const int*)(ub + o_koff);
-        ts.kld = (const int*)(ub + o_kld); ts.kbq = (const double*)(ub + o_kq); ts.ken = (const double*)(ub + o_ken);
-        ts.dEk = TS.dEk[p][1 - tcur].as<double>(); ts.betabar = betabar; ts.nops = (int)avg_ops.size();
-        ts.ops = (const double* const*)(ub + o_avp); ts.dops = tab_avg(p); ts.diag_off = (const int64_t*)(ub + o_doff);
-        launch_tan_sums(ts, TS.part.as<double>(), TS.out.as<double>() + (size_t)p * TanSumArgs::kMaxOut, c->stream);
-        d2h(c, &dl[p], TS.dlam.as<double>() + gs, sizeof(double));
-        c->launches += 14;
+        d2h(c, shp->den.data(), TS.dEall.p, sizeof(double) * NP * ns);
       }
+      // dO_new = dZ_I F Z_J^T + Z_I (F dZ_J^T + dF Z_J^T)
+      launch_update_tangents(c, tm, U, UpdateTangents{TS.dZ.as<double>(), TS.dZt.as<double>(), ys, &TS.dT, dptr,
+                                                      (double* const*)(dptr + 8)});
+      if (dm) {
+        const int64_t ncd = newops[nops_h].size;
+        for (int p = 0; p < NP; ++p) {
+          shp->dcd[p].ensure(sizeof(double) * std::max<int64_t>(ncd, 1));
+          CU(cudaMemcpyAsync(shp->dcd[p].p, op_tan(tnext, nops_h, p), sizeof(double) * ncd, cudaMemcpyDeviceToDevice,
+                             c->stream));
+        }
+      }
+      // weighted sums of the thermodynamics and operator-average tangents
+      TanSumArgs ts{};
+      ts.nstates = P.nstates; ts.state_block = (const int*)(mb + o_sb); ts.bq = (const double*)(mb + o_bq);
+      ts.en = c->en.as<double>(); ts.dE = TS.dEall.as<double>(); ts.totalS = m.totalS ? 1 : 0;
+      for (int t = 0; t < 4; ++t) ts.beta[t] = betas[t];
+      ts.nkept = nkept; ts.nkblocks = nk; ts.kstate_block = (const int*)(ub + o_ksb); ts.koff = (const int*)(ub + o_koff);
+      ts.kld = (const int*)(ub + o_kld); ts.kbq = (const double*)(ub + o_kq); ts.ken = (const double*)(ub + o_ken);
+      ts.dEk = TS.dEk[tnext].as<double>(); ts.betabar = betabar; ts.nops = (int)avg_ops.size();
+      ts.ops = (const double* const*)(ub + o_avp); ts.dops = tab_avg; ts.diag_off = (const int64_t*)(ub + o_doff);
+      launch_tan_sums(ts, TS.part.as<double>(), TS.out.as<double>(), c->stream);
+      c->launches += 6;
       d2h(c, sums.data(), TS.out.p, sizeof(double) * sums.size());
       CU(cudaStreamSynchronize(c->stream));
       check_flag(c);
@@ -3290,7 +3307,7 @@ void update_ops_impl(nrg_ctx* c, int model, const nrg_blocks* old_kept, const nr
     oldptr[o] = c->ops_a[o].as<double>();
   }
   UpdatePlan U;
-  plan_update(U, c->num_sms, m, B, P, K, oldops);
+  plan_update(U, c->num_sms, 1, m, B, P, K, oldops);
   int64_t total = 0;
   std::vector<int64_t> obase(nops);
   for (int o = 0; o < nops; ++o) {

@@ -67,7 +67,7 @@ __device__ __forceinline__ void gemm_tile(GemmSmem<RW>& S, int K, int rows, Load
   };
   fetch(0);
   for (int k0 = 0; k0 < K; k0 += kGemmK) {
-    __syncthreads();
+    __syncthreads();  // also of the CTA's last call, whose tiles S holds
 #pragma unroll
     for (int q = 0; q < kPerA; ++q) {
       const int idx = tid + q * kGemmThreads;

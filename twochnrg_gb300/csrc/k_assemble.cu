@@ -32,13 +32,16 @@ __global__ void __launch_bounds__(256) assemble_kernel(AssembleArgs A, const int
   const int NT = A.ntypes;
   const size_t PB = (size_t)NT * NT * NO * 2;
   const double* coef = A.coef + PB * b;
-  double* Hrow = A.H + A.hoff[b] + (int64_t)r * n;
+  // grid row y: direction y of a tangent pass (other old energies and operators)
+  const double* const* ops = A.ops + 8 * blockIdx.y;
+  const double* st_eold = A.st_eold + A.e_stride * blockIdx.y;
+  double* Hrow = A.H + A.h_stride * blockIdx.y + A.hoff[b] + (int64_t)r * n;
   for (int c = threadIdx.x; c < n; c += blockDim.x) {
     const int i = min(r, c), j = max(r, c);  // the reference evaluates ist <= jst
     const int gi = s0 + i, gj = s0 + j;
     double v;
     if (i == j) {
-      v = __dmul_rn(A.sqrt_lambda, A.st_eold[gi]);
+      v = __dmul_rn(A.sqrt_lambda, st_eold[gi]);
       if (A.onsite) v = __dadd_rn(v, __dmul_rn(A.eN, __dadd_rn(A.site_q[A.st_type[gi]], 1.0)));
     } else {
       const int p = A.st_seg[gi], q = A.st_seg[gj];
@@ -55,10 +58,10 @@ __global__ void __launch_bounds__(256) assemble_kernel(AssembleArgs A, const int
           // times chi_N (sign and table folded into cij, exact)
           double acc = 0.0;
           for (int o = 0; o < 2; ++o) {
-            double old = old_element(A.ops[o], A.pair_fwd[pt + o], A.pair_fwd_ld[pt + o], ai, aj);
+            double old = old_element(ops[o], A.pair_fwd[pt + o], A.pair_fwd_ld[pt + o], ai, aj);
             int dir = 0;
             if (fabs(old) < 1.e-20 || A.hc_switch[o * NT * NT + ti * NT + tj]) {
-              old = old_element(A.ops[o], A.pair_bwd[pt + o], A.pair_bwd_ld[pt + o], aj, ai);
+              old = old_element(ops[o], A.pair_bwd[pt + o], A.pair_bwd_ld[pt + o], aj, ai);
               dir = 1;
             }
             acc = __dadd_rn(acc, __dmul_rn(cij[o * 2 + dir], old));
@@ -71,27 +74,27 @@ __global__ void __launch_bounds__(256) assemble_kernel(AssembleArgs A, const int
           v = __dsub_rn(__dsub_rn(0.0, __dmul_rn(A.delta, A.sc_pair[ti * NT + tj])),
                         __dmul_rn(A.delta, A.sc_pair[tj * NT + ti]));
         } else {
-          double old = old_element(A.ops[0], A.pair_fwd[pt], A.pair_fwd_ld[pt], ai, aj);
+          double old = old_element(ops[0], A.pair_fwd[pt], A.pair_fwd_ld[pt], ai, aj);
           int dir = 0;
           if (fabs(old) < 1.e-20 || A.hc_switch[ti * NT + tj]) {
-            old = old_element(A.ops[0], A.pair_bwd[pt], A.pair_bwd_ld[pt], aj, ai);
+            old = old_element(ops[0], A.pair_bwd[pt], A.pair_bwd_ld[pt], aj, ai);
             dir = 1;
           }
           v = __dmul_rn(__dmul_rn(A.chi[0], old), cij[dir]);
         }
       } else if (A.model == 0) {
         // ((chi_N*OldEl)*CoefMatEl)*FermiSign, FermiSign folded into the table.
-        double old = old_element(A.ops[0], A.pair_fwd[pt], A.pair_fwd_ld[pt], ai, aj);
+        double old = old_element(ops[0], A.pair_fwd[pt], A.pair_fwd_ld[pt], ai, aj);
         int dir = 0;
-        if (fabs(old) < 1.e-20) { old = old_element(A.ops[0], A.pair_bwd[pt], A.pair_bwd_ld[pt], aj, ai); dir = 1; }
+        if (fabs(old) < 1.e-20) { old = old_element(ops[0], A.pair_bwd[pt], A.pair_bwd_ld[pt], aj, ai); dir = 1; }
         v = __dmul_rn(__dmul_rn(A.chi[0], old), cij[dir]);
       } else if (A.model == 1) {
         // sum over sigma of FermiSign*OldEl*fd, then times chi_N.
         double acc = 0.0;
         for (int o = 0; o < 2; ++o) {
-          double old = old_element(A.ops[o], A.pair_fwd[pt + o], A.pair_fwd_ld[pt + o], ai, aj);
+          double old = old_element(ops[o], A.pair_fwd[pt + o], A.pair_fwd_ld[pt + o], ai, aj);
           int dir = 0;
-          if (fabs(old) < 1.e-20) { old = old_element(A.ops[o], A.pair_bwd[pt + o], A.pair_bwd_ld[pt + o], aj, ai); dir = 1; }
+          if (fabs(old) < 1.e-20) { old = old_element(ops[o], A.pair_bwd[pt + o], A.pair_bwd_ld[pt + o], aj, ai); dir = 1; }
           acc = __dadd_rn(acc, __dmul_rn(cij[o * 2 + dir], old));
         }
         v = __dmul_rn(acc, A.chi[0]);
@@ -99,9 +102,9 @@ __global__ void __launch_bounds__(256) assemble_kernel(AssembleArgs A, const int
         // sum over channels and sigma of (chi_ch*OldEl_ch)*FullMatEl.
         double acc = 0.0;
         for (int ch = 0; ch < 2; ++ch) {
-          double old = old_element(A.ops[ch], A.pair_fwd[pt + ch], A.pair_fwd_ld[pt + ch], ai, aj);
+          double old = old_element(ops[ch], A.pair_fwd[pt + ch], A.pair_fwd_ld[pt + ch], ai, aj);
           int dir = 0;
-          if (fabs(old) < 1.e-20) { old = old_element(A.ops[ch], A.pair_bwd[pt + ch], A.pair_bwd_ld[pt + ch], aj, ai); dir = 1; }
+          if (fabs(old) < 1.e-20) { old = old_element(ops[ch], A.pair_bwd[pt + ch], A.pair_bwd_ld[pt + ch], aj, ai); dir = 1; }
           const double x = __dmul_rn(A.chi[ch], old);
           acc = __dadd_rn(acc, __dmul_rn(x, cij[(ch * 2 + 0) * 2 + dir]));
           acc = __dadd_rn(acc, __dmul_rn(x, cij[(ch * 2 + 1) * 2 + dir]));
@@ -136,9 +139,9 @@ void launch_unpack(const UnpackArgs& a, int nstates, cudaStream_t s) {
 }
 
 void launch_assemble(const AssembleArgs& a, int64_t total_rows, const int* row_block, const int* row_index,
-                     cudaStream_t s) {
+                     cudaStream_t s, int ndir) {
   if (total_rows <= 0) return;
-  assemble_kernel<<<(unsigned)total_rows, 256, 0, s>>>(a, row_block, row_index);
+  assemble_kernel<<<dim3((unsigned)total_rows, ndir), 256, 0, s>>>(a, row_block, row_index);
 }
 
 }  // namespace nrg

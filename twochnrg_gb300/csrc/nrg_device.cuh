@@ -179,6 +179,8 @@ struct AssembleArgs {
   const double* sc_pair;     // [ntypes^2]
   const int* hc_switch;      // [ntypes^2]; model 5: [2 * ntypes^2], spin up first
   double delta;
+  // directions of a tangent pass: strides of H and st_eold (ops: 8 pointers each)
+  int64_t h_stride, e_stride;
 };
 // Blocks from packed upper triangles; block b's at packed + poff[b].
 struct UnpackArgs {
@@ -192,7 +194,7 @@ struct UnpackArgs {
 };
 void launch_unpack(const UnpackArgs& a, int nstates, cudaStream_t s);
 void launch_assemble(const AssembleArgs& a, int64_t total_rows, const int* row_block,
-                     const int* row_index, cudaStream_t s);
+                     const int* row_index, cudaStream_t s, int ndir = 1);
 
 // ---------------------------------------------------------------- eigensolver
 struct TridiagArgs {
@@ -387,6 +389,17 @@ struct UpdateArgs {
   const int* tile1_group;
   const int* tile1_mn;
   int ntiles1, rows1;
+  // The tangent pass (ndir > 0): per direction y the tangents of Z and Zt, of T
+  // (from the terms with Zt's and the old operators' tangents) and of the
+  // operators (16 pointers per direction), O' = Z' T + Z T'.
+  int ndir;
+  const double* dZ;
+  const double* dZt;
+  int64_t z_stride;
+  double* dT;
+  int64_t t_stride;
+  const double* const* dold_ops;
+  double* const* dnew_ops;
 };
 void launch_update(const UpdateArgs& a, cudaStream_t s);
 
@@ -408,6 +421,8 @@ void launch_opdiag(const OpDiagArgs& a, const int* kstate_block, int nk, double*
 int reduce_partial_count();
 
 // ---------------------------------------------------------------- tangents (k_tangent.cu)
+// Arrays of the tangent pass hold its kTanDirs directions one after the other.
+constexpr int kTanDirs = 4;
 struct TanEigArgs {      // per block: dlambda = diag(dH~), C = dH~_kl / (lambda_l - lambda_k)
   const int* bsize;
   const int* soff;
@@ -419,13 +434,14 @@ struct TanEigArgs {      // per block: dlambda = diag(dH~), C = dH~_kl / (lambda
   double* C;
   double* dlam;          // per state
   double degen_tol;      // relative gap below which two levels do not couple
+  int64_t h_stride, c_stride;
+  int nstates;
 };
 void launch_tan_eig(const TanEigArgs& a, int nblocks, cudaStream_t s);
+// gs_out: each direction's dlam[gs].
 void launch_tan_shift(const double* dlam, int nstates, int gs, double* dE_all, const int* kept_state, int nkept,
-                      double* dE_kept, cudaStream_t s);
-void launch_tan_gather(const double* dE_kept_old, const int* stcf, int n, double* out, cudaStream_t s);
-void launch_tan_axpy3(const double* a, const double* b, const double* c, double scale, int64_t n, double* out,
-                      cudaStream_t s);
+                      double* dE_kept, double* gs_out, cudaStream_t s);
+void launch_tan_gather(const double* dE_kept_old, int nold, const int* stcf, int n, double* out, cudaStream_t s);
 void launch_tan_scale(const double* a, double scale, int64_t n, double* out, cudaStream_t s);
 struct TanSumArgs {      // weighted sums of the thermodynamics and operator-average tangents
   static constexpr int kMaxOut = 24;  // 12 thermo sums, 2 per operator (<= 5), the last: sum deg w dE (kept)
@@ -446,7 +462,7 @@ struct TanSumArgs {      // weighted sums of the thermodynamics and operator-ave
   double betabar;
   int nops;
   const double* const* ops;   // averaged operators (primal) and their tangents
-  const double* const* dops;
+  const double* const* dops;  // 8 per direction
   const int64_t* diag_off;    // [nops * nkblocks]
 };
 size_t tan_partial_doubles();
