@@ -65,6 +65,21 @@ struct DevBuf {
   template <class T> T* as() const { return reinterpret_cast<T*>(p); }
 };
 
+// Page-locked host memory for results read back.
+struct PinBuf {
+  void* p = nullptr;
+  size_t cap = 0;
+  ~PinBuf() { if (p) cudaFreeHost(p); }
+  void ensure(size_t bytes) {
+    if (bytes <= cap) return;
+    const size_t want = std::max(bytes, cap + cap / 2);
+    if (p) { CU(cudaFreeHost(p)); p = nullptr; cap = 0; }
+    CU(cudaMallocHost(&p, want));
+    cap = want;
+  }
+  template <class T> T* as() const { return reinterpret_cast<T*>(p); }
+};
+
 // Packs host arrays into one staging buffer and one device buffer so a table
 // set costs a single host-to-device copy.
 struct Packer {
@@ -175,6 +190,7 @@ struct nrg_ctx {
   cudaEvent_t span_join = nullptr;
   cudaEvent_t rows_fork = nullptr, rows_join = nullptr;
   nrg::DevBuf gpart_k[kMaxSplit], gbig, rlist, slist, swork;
+  nrg::PinBuf pin, pin_avg;            // results of a read_back; operator averages of the last two iterations
   // mixed precision: per concurrent grid the blocked reduction's [V W], column
   // and share scratch, and the tensor-core product's slices
   nrg::DevBuf pvw[kMaxSplit], pcol[kMaxSplit], ppart[kMaxSplit], ozk[kMaxSplit];
@@ -287,14 +303,45 @@ void stream_wait(nrg_ctx* c) {
   CU(cudaEventSynchronize(c->bsync));
 }
 
-void check_flag(nrg_ctx* c) {
-  int f = 0;
-  CU(cudaMemcpy(&f, c->flag.p, sizeof(int), cudaMemcpyDeviceToHost));
+void check_flag_value(int f) {
   if (f & DEV_SIZE) throw NrgError(NRG_ERR_SIZE, "a block exceeds the eigensolver size limit");
   if (f & DEV_DEGEN_OVERFLOW) throw NrgError(NRG_ERR_SIZE, "too many near-degenerate levels for SetDegen");
   if (f & DEV_BAD_INPUT) throw NrgError(NRG_ERR_ARG, "non-finite value met in an eigenvalue solve");
   if (f & DEV_NOT_CONVERGED) throw NrgError(NRG_ERR_NOT_CONVERGED, "inverse iteration did not converge");
   if (f & DEV_TIMEOUT) throw NrgError(NRG_ERR_TIMEOUT, "a kernel's bounded wait gave up");
+}
+void check_flag(nrg_ctx* c) {
+  int f = 0;
+  CU(cudaMemcpy(&f, c->flag.p, sizeof(int), cudaMemcpyDeviceToHost));
+  check_flag_value(f);
+}
+
+// Device results to the host with the flag and one wait for the stream: the copies
+// go to page-locked memory, where each runs on behind the kernels (a copy to
+// pageable memory holds the host until it is done, and the flag's own was another
+// round trip).
+struct ReadItem { void* dst; const void* src; size_t bytes; };
+void read_back(nrg_ctx* c, std::initializer_list<ReadItem> items) {
+  size_t n = 16;
+  for (const ReadItem& it : items) n += (it.bytes + 15) & ~size_t(15);
+  c->pin.ensure(n);
+  char* h = c->pin.as<char>();
+  CU(cudaMemcpyAsync(h, c->flag.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  size_t at = 16;
+  for (const ReadItem& it : items) {
+    if (it.bytes) CU(cudaMemcpyAsync(h + at, it.src, it.bytes, cudaMemcpyDeviceToHost, c->stream));
+    at += (it.bytes + 15) & ~size_t(15);
+    c->timing.d2h_bytes += (int64_t)it.bytes;
+  }
+  stream_wait(c);
+  int f;
+  std::memcpy(&f, h, sizeof(int));
+  check_flag_value(f);
+  at = 16;
+  for (const ReadItem& it : items) {
+    if (it.bytes) std::memcpy(it.dst, h + at, it.bytes);
+    at += (it.bytes + 15) & ~size_t(15);
+  }
 }
 
 // ------------------------------------------------------------------ eigensolve
@@ -1574,13 +1621,32 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
   // N = 0 and as ScaleFactor(N-1) * Delta_SC = Lambda^((N-1)/2) / HLF *
   // Delta_SC after that (NRG_main.cpp:220-227, 276, 414-419).
   const bool sc = m.kind == MODEL_1CHS || m.kind == MODEL_1CHSZ;
-  cudaEvent_t it0, it1;
-  CU(cudaEventCreate(&it0));
-  CU(cudaEventCreateWithFlags(&it1, c->shared_gpu ? cudaEventBlockingSync : cudaEventDefault));
-  EvGuard itg{it0, it1};
+  cudaEvent_t it0[2], it1[2];
+  for (int k = 0; k < 2; ++k) { CU(cudaEventCreate(&it0[k])); CU(cudaEventCreate(&it1[k])); }
+  EvGuard itg0{it0[0], it1[0]}, itg1{it0[1], it1[1]};
+  // What of an iteration is read when the stream is next waited for: the operator
+  // averages, its times (the host's: since the iteration before was finished).
+  c->pin_avg.ensure(sizeof(double) * 16);
+  int last_N = -1;
+  size_t last_avg = 0;
+  auto t_last = clock::now();
+  auto finish_last = [&] {
+    tm.collect();
+    if (last_N < 0) return;
+    IterResult& R = c->iters.back();
+    const double* avg = c->pin_avg.as<double>() + 8 * (last_N & 1);
+    const double Zk = avg[last_avg];
+    for (size_t k = 0; k < last_avg; ++k) R.opavg.push_back(std::fabs(Zk) < 1.e-20 ? avg[k] : avg[k] / Zk);
+    float ms = 0.f;
+    CU(cudaEventElapsedTime(&ms, it0[last_N & 1], it1[last_N & 1]));
+    R.device_ms = ms;
+    const auto now = clock::now();
+    R.wall_ms = std::chrono::duration<double, std::milli>(now - t_last).count();
+    t_last = now;
+    last_N = -1;
+  };
   for (int N = N0; N < cfg->nsites; ++N) {
-    const auto t_iter = clock::now();
-    CU(cudaEventRecord(it0, c->stream));
+    CU(cudaEventRecord(it0[N & 1], c->stream));
     IterResult R;
     eN = onsite(N);
     const double delta = !sc ? 0.0 : (N == 0 ? cfg->delta_sc
@@ -1633,12 +1699,10 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
     c->launches += 4;
     std::vector<double> scal(20);
     R.en.resize(P.nstates);
-    d2h(c, scal.data(), c->scal.p, sizeof(double) * 20);
-    d2h(c, keptb.data(), bs.kept, sizeof(int) * nb);
-    d2h(c, R.en.data(), c->en.p, sizeof(double) * P.nstates);
     tm.stop(tc, &c->timing.cut_ms);
-    stream_wait(c);
-    check_flag(c);
+    read_back(c, {{scal.data(), c->scal.p, sizeof(double) * 20}, {keptb.data(), bs.kept, sizeof(int) * nb},
+                  {R.en.data(), c->en.p, sizeof(double) * P.nstates}});
+    finish_last();
     R.emin = scal[0]; R.ecut = scal[1]; R.nkept = (int)scal[2];
     R.qn = B.blk.qn; R.bsize = P.bsize;
     for (int t = 0; t < 4; ++t) {
@@ -1719,18 +1783,13 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
     od.diag_off = (const int64_t*)(ub + o_doff); od.out = c->scal.as<double>() + 24;
     launch_opdiag(od, (const int*)(ub + o_ksb), (int)kstate_block.size(), c->partial.as<double>(), c->stream);
     c->launches += 2;
-    std::vector<double> avg(8);
-    d2h(c, avg.data(), c->scal.as<double>() + 24, sizeof(double) * 8);
+    // The averages are read with the next iteration's results (finish_last), so
+    // that the host builds that iteration's tables while this one's eigenvectors
+    // and operators are computed.
+    double* const avg = c->pin_avg.as<double>() + 8 * (N & 1);
+    CU(cudaMemcpyAsync(avg, c->scal.as<double>() + 24, sizeof(double) * 8, cudaMemcpyDeviceToHost, c->stream));
+    c->timing.d2h_bytes += (int64_t)sizeof(double) * 8;
     tm.stop(to, &c->timing.cut_ms);
-    stream_wait(c);
-    check_flag(c);
-    tm.collect();
-    const double Zk = avg[avg_ops.size()];
-    for (size_t k = 0; k < avg_ops.size(); ++k) {
-      double s = avg[k];
-      if (!(std::fabs(Zk) < 1.e-20)) s = s / Zk;
-      R.opavg.push_back(s);
-    }
     // ---------------- tangents of this iteration (nrg_grad_forward)
     std::unique_ptr<DmShell> shp;
     if (dm) shp = std::make_unique<DmShell>();
@@ -1872,10 +1931,7 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
       ts.ops = (const double* const*)(ub + o_avp); ts.dops = tab_avg; ts.diag_off = (const int64_t*)(ub + o_doff);
       launch_tan_sums(ts, TS.part.as<double>(), TS.out.as<double>(), c->stream);
       c->launches += 6;
-      d2h(c, sums.data(), TS.out.p, sizeof(double) * sums.size());
-      CU(cudaStreamSynchronize(c->stream));
-      check_flag(c);
-      tm.collect();
+      read_back(c, {{sums.data(), TS.out.p, sizeof(double) * sums.size()}});
       // derivatives of the reported values from the sums (CalcSuscep,
       // CalcEntropy and CalcOpAvg differentiated: d e^{-beta E} = -beta e^{-beta E} dE)
       for (int p = 0; p < NP; ++p) {
@@ -1928,16 +1984,15 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
     S.ops = newops;
     S.cur = nxt;
     for (int ich = 0; ich < m.nchan; ++ich) chi[ich] = hop(N);
-    CU(cudaEventRecord(it1, c->stream));
-    CU(cudaEventSynchronize(it1));
-    float it_ms = 0.f;
-    CU(cudaEventElapsedTime(&it_ms, it0, it1));
-    R.device_ms = it_ms;
-    R.wall_ms = std::chrono::duration<double, std::milli>(clock::now() - t_iter).count();
+    CU(cudaEventRecord(it1[N & 1], c->stream));
     c->iters.push_back(std::move(R));
+    last_N = N;
+    last_avg = avg_ops.size();
   }
   CU(cudaEventRecord(span1, c->stream));
   CU(cudaEventSynchronize(span1));
+  check_flag(c);
+  finish_last();
   float span_ms = 0.f;
   CU(cudaEventElapsedTime(&span_ms, span0, span1));
   c->timing.device_ms = span_ms;
@@ -3006,14 +3061,11 @@ void diag_blocks_impl(nrg_ctx* c, int nb, const int* sizes, const double* packed
   run_tridiag_and_bisect(c, tm, P, order, (const int*)(mb + o_order), (const int*)(mb + o_bsize),
                          (const int64_t*)(mb + o_hoff), (const int*)(mb + o_soff), (const int*)(mb + o_sb));
   std::vector<double> ev(P.nstates);
-  d2h(c, ev.data(), c->ev.p, sizeof(double) * P.nstates);
-  CU(cudaStreamSynchronize(c->stream));
-  check_flag(c);
+  read_back(c, {{ev.data(), c->ev.p, sizeof(double) * P.nstates}});
   P.nvec = bs;
   run_vectors(c, tm, P, ev, (const int*)(mb + o_bsize), (const int64_t*)(mb + o_hoff), (const int*)(mb + o_soff));
   d2h(c, evecs, c->Z.p, sizeof(double) * (size_t)P.ysize);
-  CU(cudaStreamSynchronize(c->stream));
-  check_flag(c);
+  read_back(c, {});
   tm.collect();
   std::memcpy(evals, ev.data(), sizeof(double) * P.nstates);
 }
@@ -3138,14 +3190,11 @@ void diag_hn_impl(nrg_ctx* c, int model, const double* params, int nparams, cons
   run_tridiag_and_bisect(c, tm, P, AT.order, (const int*)(mb + AT.o_order), (const int*)(mb + AT.o_bsize),
                          (const int64_t*)(mb + AT.o_hoff), (const int*)(mb + AT.o_soff), (const int*)(mb + AT.o_sb));
   std::vector<double> ev(P.nstates);
-  d2h(c, ev.data(), c->ev.p, sizeof(double) * P.nstates);
-  CU(cudaStreamSynchronize(c->stream));
-  check_flag(c);
+  read_back(c, {{ev.data(), c->ev.p, sizeof(double) * P.nstates}});
   P.nvec = P.bsize;
   run_vectors(c, tm, P, ev, AT.aa.bsize, AT.aa.hoff, AT.aa.bstate);
   d2h(c, evec_out, c->Z.p, sizeof(double) * (size_t)P.ysize);
-  CU(cudaStreamSynchronize(c->stream));
-  check_flag(c);
+  read_back(c, {});
   tm.collect();
   // SetE0zero (NRGarrayClass.cpp:234-241).
   const double emin = *std::min_element(ev.begin(), ev.end());
