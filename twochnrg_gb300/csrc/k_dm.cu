@@ -48,16 +48,18 @@ __global__ void __launch_bounds__(kGemmThreads, 6) gemm_jobs_kernel(const GemmJo
   }
 }
 
-// One CTA per block of shell N.  Kept x kept elements are the SU(2)-weighted
+// kTraceParts CTAs per block of shell N (one per block: 100 us at 500 kept, 34
+// blocks of up to 232 states; 14 us so).  Kept x kept elements are the SU(2)-weighted
 // sums over the block's child terms, evaluated for i <= j and mirrored (the
 // reference fills the upper triangle); a discarded state's diagonal is its
 // FDM Boltzmann weight; everything else is zero.
+constexpr int kTraceParts = 16;
 __global__ void __launch_bounds__(256) dm_trace_kernel(DmTraceArgs A) {
   const int b = blockIdx.x;
   const int n = A.bsize[b], k = A.nkept[b], s0 = A.soff[b];
   const int t0 = A.term_first[b], nt = A.term_count[b];
   double* R = A.rho + A.roff[b];
-  for (int64_t idx = threadIdx.x; idx < (int64_t)n * n; idx += blockDim.x) {
+  for (int64_t idx = blockIdx.y * blockDim.x + threadIdx.x; idx < (int64_t)n * n; idx += gridDim.y * blockDim.x) {
     const int i = (int)(idx / n), j = (int)(idx - (int64_t)i * n);
     const int ii = i < j ? i : j, jj = i < j ? j : i;
     double v = 0.0;
@@ -468,7 +470,7 @@ void launch_gemm_jobs(const GemmJob* jobs, const int* tile_job, const int* tile_
 }
 
 void launch_dm_trace(const DmTraceArgs& a, int nblocks, cudaStream_t s) {
-  if (nblocks > 0) dm_trace_kernel<<<nblocks, 256, 0, s>>>(a);
+  if (nblocks > 0) dm_trace_kernel<<<dim3(nblocks, kTraceParts), 256, 0, s>>>(a);
 }
 
 void launch_dm_records(const DmRecArgs& a, int pass, cudaStream_t s) {
