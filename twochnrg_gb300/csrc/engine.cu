@@ -62,6 +62,7 @@ struct DevBuf {
     CU(cudaMalloc(&p, want));
     cap = want;
   }
+  void take(DevBuf& o) { std::swap(p, o.p); std::swap(cap, o.cap); }
   template <class T> T* as() const { return reinterpret_cast<T*>(p); }
 };
 
@@ -143,6 +144,13 @@ struct DmShell {
   std::vector<double> den;             // [p * nstates + i]: d en
   DevBuf dZ[4], dcd[4], drho[4];       // d Z (rows, the layout of Z), d c_d, d rho (the layout of rho)
   DevBuf ltpart;                       // tangent Lehmann partial sums, [p][the layout of lpart]
+  // The device memory of a shell of the sweep before.
+  void reuse(DmShell& o, bool tan) {
+    Z.take(o.Z); cdel.take(o.cdel); rho.take(o.rho); lpart.take(o.lpart);
+    if (!tan) return;
+    for (int p = 0; p < 4; ++p) { dZ[p].take(o.dZ[p]); dcd[p].take(o.dcd[p]); drho[p].take(o.drho[p]); }
+    ltpart.take(o.ltpart);
+  }
 };
 
 struct IterResult {
@@ -190,6 +198,8 @@ struct nrg_ctx {
   cudaEvent_t span_join = nullptr;
   cudaEvent_t rows_fork = nullptr, rows_join = nullptr;
   nrg::DevBuf gpart_k[kMaxSplit], gbig, rlist, slist, swork;
+  nrg::PinBuf stage;                   // tables on their way to the device
+  size_t stage_at = 0;
   nrg::PinBuf pin, pin_avg;            // results of a read_back; operator averages of the last two iterations
   // mixed precision: per concurrent grid the blocked reduction's [V W], column
   // and share scratch, and the tensor-core product's slices
@@ -205,6 +215,10 @@ struct nrg_ctx {
   bool shared_gpu = false;  // a batch worker: other contexts run beside this one
   cudaEvent_t bsync = nullptr;  // blocking-sync event of stream_wait
   std::vector<std::unique_ptr<nrg::DmShell>> dm;
+  // While a sweep that keeps shells runs: the shells of the one before, whose
+  // device memory the new ones take over (40 shells' allocations and frees took
+  // 12 of a DM-NRG pass of 110 ms at 500 kept).  What is left is freed at its end.
+  std::vector<std::unique_ptr<nrg::DmShell>> dm_spare;
   bool dm_rho_valid = false;
   bool dm_drho_valid = false;          // the density matrices' tangents are built too
   nrg::DevBuf dmtan;                   // scratch of the tangent rotations and rho.A products
@@ -278,9 +292,22 @@ struct Timer {
 };
 
 // Stream-ordered copies that also count the bytes crossing the host boundary.
-void h2d(nrg_ctx* c, void* dst, const void* src, size_t bytes, cudaStream_t s = nullptr) {
+// Tables of more than 64 KB go up from page-locked memory, one after the other
+// until the stream is next waited for: from pageable memory they would hold the
+// host until the stream is there.  Smaller ones travel with the launches, which is
+// faster than a copy engine (a (Q,Sz) sweep at 60 kept 5.05 ms, 5.4 staged); what
+// does not fit goes directly.
+constexpr size_t kStageBytes = (size_t)4 << 20, kStageFrom = (size_t)64 << 10;
+void h2d(nrg_ctx* c, void* dst, const void* src, size_t bytes) {
   if (!bytes) return;
-  CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s ? s : c->stream));
+  if (bytes > kStageFrom) c->stage.ensure(kStageBytes);
+  if (bytes > kStageFrom && c->stage_at + bytes <= kStageBytes) {
+    void* at = c->stage.as<char>() + c->stage_at;
+    std::memcpy(at, src, bytes);
+    src = at;
+    c->stage_at += (bytes + 255) & ~size_t(255);
+  }
+  CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream));
   c->timing.h2d_bytes += (int64_t)bytes;
 }
 void d2h(nrg_ctx* c, void* dst, const void* src, size_t bytes) {
@@ -296,11 +323,13 @@ void d2h(nrg_ctx* c, void* dst, const void* src, size_t bytes) {
 void stream_wait(nrg_ctx* c) {
   if (!c->shared_gpu) {
     CU(cudaStreamSynchronize(c->stream));
+    c->stage_at = 0;
     return;
   }
   if (!c->bsync) CU(cudaEventCreateWithFlags(&c->bsync, cudaEventBlockingSync | cudaEventDisableTiming));
   CU(cudaEventRecord(c->bsync, c->stream));
   CU(cudaEventSynchronize(c->bsync));
+  c->stage_at = 0;
 }
 
 void check_flag_value(int f) {
@@ -811,6 +840,26 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
   if (nspan > 0)  // two cooperative kernels at once might each get part of the SMs
     for (int k = 0; K > 1 && k < K; ++k) CU(cudaStreamWaitEvent(c->stream, c->join[k], 0));
   const bool both = nspan + nmid > 0 && nrows0 < nb;
+  // The row kernel's lists, up before the streams fork: it has to be the first.
+  int kclusters = 0;
+  size_t o_list = 0, o_first = 0;
+  if (nrows0 < nb) {
+    kclusters = std::min({rncl, nb - nrows0, nspan > 0 ? std::max(1, sp.rows_clusters) : rncl});
+    std::vector<double> cst(nb);
+    std::vector<int> bin, list, first;
+    for (int q = nrows0; q < nb; ++q) cst[q] = rows_cost(P.bsize[order_h[q]]);
+    deal_greedy(cst, nrows0, nb, kclusters, &bin);
+    for (int q = 0; q < kclusters; ++q) {
+      first.push_back((int)list.size());
+      for (int i = nrows0; i < nb; ++i)
+        if (bin[i - nrows0] == q) list.push_back(order_h[i]);
+    }
+    first.push_back((int)list.size());
+    Packer pk;
+    o_list = pk.add(list); o_first = pk.add(first);
+    c->rlist.ensure(pk.host.size() + 256);
+    h2d(c, c->rlist.p, pk.host.data(), pk.host.size());
+  }
   if (both) {
     if (!c->rows_stream) {
       CU(cudaStreamCreateWithFlags(&c->rows_stream, cudaStreamNonBlocking));
@@ -822,25 +871,10 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
   }
   auto launch_rows = [&](cudaStream_t s) {
     TridiagArgs ts = ta;
-    const int k = std::min({rncl, nb - nrows0, nspan > 0 ? std::max(1, sp.rows_clusters) : rncl});
-    std::vector<double> cst(nb);
-    std::vector<int> bin, list, first;
-    for (int q = nrows0; q < nb; ++q) cst[q] = rows_cost(P.bsize[order_h[q]]);
-    deal_greedy(cst, nrows0, nb, k, &bin);
-    for (int q = 0; q < k; ++q) {
-      first.push_back((int)list.size());
-      for (int i = nrows0; i < nb; ++i)
-        if (bin[i - nrows0] == q) list.push_back(order_h[i]);
-    }
-    first.push_back((int)list.size());
-    Packer pk;
-    const size_t o_list = pk.add(list), o_first = pk.add(first);
-    c->rlist.ensure(pk.host.size() + 256);
-    h2d(c, c->rlist.p, pk.host.data(), pk.host.size(), s);
     ts.order = (const int*)(c->rlist.as<char>() + o_list); ts.first = (const int*)(c->rlist.as<char>() + o_first);
     ts.nblocks = nb - nrows0;
     ts.maxn = std::max(P.bsize[order_h[nrows0]], 2);
-    CU(launch_tridiag_rows(ts, rcl, k, s));
+    CU(launch_tridiag_rows(ts, rcl, kclusters, s));
     c->launches++; c->timing.tridiag_launches++;
   };
   // Beside the span kernel the row kernel goes first: its clusters of 16 need SMs
@@ -1487,6 +1521,7 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
     S.m.op_avg = {0, 0, 0};
   }
   if (dm) {
+    c->dm_spare = std::move(c->dm);
     c->dm.clear();
     c->dm_rho_valid = false;
     c->dm_drho_valid = false;
@@ -1792,7 +1827,10 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
     tm.stop(to, &c->timing.cut_ms);
     // ---------------- tangents of this iteration (nrg_grad_forward)
     std::unique_ptr<DmShell> shp;
-    if (dm) shp = std::make_unique<DmShell>();
+    if (dm) {
+      shp = std::make_unique<DmShell>();
+      if (c->dm.size() < c->dm_spare.size()) shp->reuse(*c->dm_spare[c->dm.size()], tan != nullptr);
+    }
     if (tan) {
       TangentState& TS = *tan;
       const int NP = TangentState::NP;
@@ -1993,6 +2031,7 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
   CU(cudaEventSynchronize(span1));
   check_flag(c);
   finish_last();
+  c->dm_spare.clear();
   float span_ms = 0.f;
   CU(cudaEventElapsedTime(&span_ms, span0, span1));
   c->timing.device_ms = span_ms;
@@ -2260,11 +2299,9 @@ void dm_backprop_impl(nrg_ctx* c, const nrg_dm_params* prm, double* rho_trace) {
       launch_dm_trace(tt, nbN, c->stream);
       c->launches++;
     }
-    CU(cudaStreamSynchronize(c->stream));  // meta and T are reused by the next shell
   }
   tm.stop(t0, &c->timing.dm_backprop_ms);
-  CU(cudaStreamSynchronize(c->stream));
-  check_flag(c);
+  read_back(c, {});
   tm.collect();
   c->dm_rho_valid = true;
   c->dm_drho_valid = tg;
@@ -2274,7 +2311,7 @@ void dm_backprop_impl(nrg_ctx* c, const nrg_dm_params* prm, double* rho_trace) {
       const DmShell& s = *c->dm[N];
       std::vector<double> R((size_t)std::max<int64_t>(s.zsize, 1));
       d2h(c, R.data(), s.rho.p, sizeof(double) * s.zsize);
-      CU(cudaStreamSynchronize(c->stream));
+      stream_wait(c);
       double t = 0.0;
       for (size_t b = 0; b < s.bsize.size(); ++b) {
         const int n = s.bsize[b];
@@ -2493,7 +2530,7 @@ void lehmann_impl(nrg_ctx* c, const nrg_dm_params* prm, int nomega, const double
     c->launches += 2;
     int64_t tot[4];
     d2h(c, tot, a.totals, sizeof(tot));
-    CU(cudaStreamSynchronize(c->stream));
+    stream_wait(c);
     int64_t nrec = 0;
     for (int Lk = 0; Lk < 4; ++Lk) nrec += tot[Lk];
     const int per_rec = tg ? 2 + 2 * NP : 2;  // key, w (and per parameter d w, 2 w d key)
@@ -2684,7 +2721,6 @@ void lehmann_impl(nrg_ctx* c, const nrg_dm_params* prm, int nomega, const double
         c->launches++;
       }
     }
-    CU(cudaStreamSynchronize(c->stream));  // meta, vmeta, dmrec and Y are reused by the next shell
   }
   // A(omega): every frequency's window shells in order.
   std::vector<int> fold_list((size_t)nw_ * window * 2, -1), fold_pos((size_t)nw_ * window * 2, 0);
@@ -2725,8 +2761,7 @@ void lehmann_impl(nrg_ctx* c, const nrg_dm_params* prm, int nomega, const double
   std::vector<double> A((size_t)nout_sets * nw_);
   d2h(c, A.data(), la.out, sizeof(double) * nout_sets * nw_);
   tm.stop(t0, &c->timing.dm_spectral_ms);
-  CU(cudaStreamSynchronize(c->stream));
-  check_flag(c);
+  read_back(c, {});
   tm.collect();
   c->timing.lehmann_pairs = nrec_all;
   c->timing.lehmann_evals = evals;
@@ -2784,7 +2819,7 @@ void dm_save_bin_impl(nrg_ctx* c, const char* dir, const char* name) {
     std::vector<double> Z((size_t)std::max<int64_t>(s.zsize, 1)), el((size_t)std::max<int64_t>(s.cd.size, 1));
     d2h(c, Z.data(), s.Z.p, sizeof(double) * s.zsize);
     d2h(c, el.data(), s.cdel.p, sizeof(double) * s.cd.size);
-    CU(cudaStreamSynchronize(c->stream));
+    stream_wait(c);
     std::vector<int> map, mbe;
     for (size_t k = 0; k < s.cd.bi.size(); ++k) {
       map.push_back(s.cd.bi[k]);
@@ -2926,7 +2961,7 @@ void dm_load_bin_impl(nrg_ctx* c, const char* dir, const char* name, int nshells
     h2d(c, sh->Z.p, fa.evec.data(), sizeof(double) * z);
     sh->cdel.ensure(sizeof(double) * std::max<int64_t>(nel, 1));
     h2d(c, sh->cdel.p, fm.mat_el.data(), sizeof(double) * nel);
-    CU(cudaStreamSynchronize(c->stream));
+    stream_wait(c);
     sh->basis = std::move(B);
     c->dm.push_back(std::move(sh));
     prev = kept;
@@ -3248,8 +3283,7 @@ void cut_states_impl(nrg_ctx* c, const nrg_blocks* aeig, const double* en, const
   d2h(c, keptb.data(), bs.kept, sizeof(int) * nb);
   d2h(c, c->out_en.data(), c->en.p, sizeof(double) * ns);
   tm.stop(tc, &c->timing.cut_ms);
-  CU(cudaStreamSynchronize(c->stream));
-  check_flag(c);
+  read_back(c, {});
   tm.collect();
   const double ecut = scal[1];
   c->out_kept.assign(ns, 0);
@@ -3371,8 +3405,7 @@ void update_ops_impl(nrg_ctx* c, int model, const nrg_blocks* old_kept, const nr
   c->out_el.resize((size_t)std::max<int64_t>(total, 1));
   for (int o = 0; o < nops; ++o)
     d2h(c, c->out_el.data() + obase[o], newptr[o], sizeof(double) * U.newops[o].size);
-  CU(cudaStreamSynchronize(c->stream));
-  check_flag(c);
+  read_back(c, {});
   tm.collect();
   c->out_map.clear(); c->out_mbe.clear();
   std::vector<size_t> mbase(nops);
