@@ -935,6 +935,7 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
   ea.split = c->spl.as<unsigned char>();
   ea.mixed_n = mixed ? std::max(thr, mixed_block_threshold()) : 0;
   cudaEvent_t t1 = tm.start();
+  for (int n : P.bsize) ea.rows2 += (int64_t)n * n;
   launch_bisect(ea, d_state_block, c->stream);
   c->launches += 3;  // FP32 copies, levels, ordering
   tm.stop(t1, &c->timing.tridiag_eig_ms);

@@ -133,7 +133,7 @@ extern "C" nrg_status nrg_diag_block_noalloc(int n, const double* a, double* eig
   if (launch_tridiag_rows(ta, cl, 1, s) != cudaSuccess) return NRG_ERR_CUDA;
   TdEigArgs ea{};
   ea.nblocks = 1; ea.bsize = L.bsize; ea.soff = L.soff; ea.d = L.d; ea.e = L.e; ea.ev = L.ev; ea.nstates = n;
-  ea.flag = L.flag; ea.maxn = n; ea.fde = L.fde; ea.e2 = L.e2; ea.split = L.split;
+  ea.flag = L.flag; ea.maxn = n; ea.rows2 = (int64_t)n * n; ea.fde = L.fde; ea.e2 = L.e2; ea.split = L.split;
   launch_bisect(ea, L.state_block, s);
   if (cudaGetLastError() != cudaSuccess) return NRG_ERR_CUDA;
   cluster_kernel<<<1, 32, 0, s>>>(L, n);

@@ -254,6 +254,7 @@ struct TdEigArgs {
   int nstates;
   int* flag;
   int maxn;              // largest block (sizes the sort's shared memory)
+  int64_t rows2;         // sum of the blocks' sizes squared: rows of all levels' passes
   float* fde;            // scratch [2*nstates]: FP32 copies of d and e for the FP32 bracket
   double* e2;            // scratch [nstates]: e^2
   unsigned char* split;  // scratch [nstates]: e_i negligible (the pieces' ends)
