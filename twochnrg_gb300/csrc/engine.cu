@@ -967,7 +967,16 @@ void run_vectors(nrg_ctx* c, Timer& tm, EigPlan& P, const std::vector<double>& e
     m = std::max(m, P.bsize[b]);
     if (P.bsize[b] <= gmax) gvecs += P.nvec[b];
   }
-  const int gw = gvecs < 8 * c->num_sms ? 4 : 8;
+  // Two warps per vector where the vectors, counted by the longest's length, leave
+  // every one two sub-partitions and the blocks are long enough for that to pay
+  // for the second exchange per group: two channels at 300 kept (blocks to 677
+  // states) 10.0 -> 7.5 ms, one channel at 500 kept (232) 6.2 either way, at 300
+  // kept (140) 2.0 -> 2.4.
+  int64_t glen = 0;
+  for (int b = 0; b < nb; ++b)
+    if (P.bsize[b] <= gmax) glen += (int64_t)P.nvec[b] * P.bsize[b];
+  const int gsplit = gmaxn >= 300 && 2 * glen <= 4 * (int64_t)c->num_sms * gmaxn ? 2 : 1;
+  const int gw = gsplit > 1 ? 2 : gvecs < 8 * c->num_sms ? 4 : 8;
   const int bw = backtransform_warps(lmaxn);
   for (int b = 0; b < nb; ++b) {
     const int n = P.bsize[b], k = P.nvec[b];
@@ -1029,7 +1038,7 @@ void run_vectors(nrg_ctx* c, Timer& tm, EigPlan& P, const std::vector<double>& e
     ba.grp_first = (const int*)(base + o_pf); ba.factors = c->bfac.as<double>();
     launch_back_factors(ba, (int)grpb.size(), c->stream);
     CU(launch_backtransform_grouped(ba, (const int*)(base + o_gb), (const int*)(base + o_gf), (int)gtab.size(), gw,
-                                    c->stream));
+                                    gsplit, c->stream));
     c->launches += 2;
   }
   tm.stop(t1, &c->timing.backtransform_ms);

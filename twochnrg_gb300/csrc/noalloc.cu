@@ -150,7 +150,7 @@ extern "C" nrg_status nrg_diag_block_noalloc(int n, const double* a, double* eig
   ba.grp_block = L.cta_block; ba.grp_index = L.grp_index; ba.grp_first = L.cta_block;  // one block: all 0
   ba.factors = L.factors;
   launch_back_factors(ba, backtransform_groups(n), s);
-  if (launch_backtransform_grouped(ba, L.cta_block, L.cta_first, (n + bw - 1) / bw, bw, s) != cudaSuccess)
+  if (launch_backtransform_grouped(ba, L.cta_block, L.cta_first, (n + bw - 1) / bw, bw, 1, s) != cudaSuccess)
     return NRG_ERR_CUDA;
   if (cudaMemcpyAsync(eigvals, L.ev, sizeof(double) * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
     return NRG_ERR_CUDA;

@@ -303,14 +303,15 @@ struct BackArgs {
   const int* grp_first;   // [blocks]
   double* factors;
 };
-// Blocks up to backtransform_grouped_max(warps) states fit the grouped kernel
-// (groups of reflectors) with that many vectors per CTA.
+// Blocks up to backtransform_grouped_max(vectors) states fit the grouped kernel
+// (groups of reflectors) with that many vectors per CTA, `split` (1 or 2) warps on
+// each.
 constexpr int kBackGroup = 4;
 int backtransform_grouped_max(int warps);
 int backtransform_groups(int n);    // groups of an n-state block
 void launch_back_factors(const BackArgs& a, int ngroups, cudaStream_t s);
 cudaError_t launch_backtransform_grouped(const BackArgs& a, const int* cta_block, const int* cta_first, int nctas,
-                                         int warps, cudaStream_t s);
+                                         int vectors, int split, cudaStream_t s);
 cudaError_t launch_backtransform(const BackArgs& a, const int* cta_block, const int* cta_first, int nctas,
                                  cudaStream_t s);
 size_t backtransform_smem_bytes(int maxn);
