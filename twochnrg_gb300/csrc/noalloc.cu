@@ -88,19 +88,38 @@ __global__ void setup_kernel(Layout L, int n, const double* a, int bw) {
 }
 
 // Clusters of close eigenvalues (gap below 1e-4 of the largest magnitude), as
-// the host forms them for nrg_diag_blocks; unused entries get count 0.
-__global__ void cluster_kernel(Layout L, int n) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  double mx = 0.0;
-  for (int i = 0; i < n; ++i) mx = fmax(mx, fabs(L.ev[i]));
+// the host forms them for nrg_diag_blocks; unused entries get count 0.  A thread
+// per level (one thread for all took 14 us at 64 states, 3.4 so).
+constexpr int kClusterThreads = 256;
+static_assert(kN <= kClusterThreads, "a thread per level");
+__global__ void __launch_bounds__(kClusterThreads) cluster_kernel(Layout L, int n) {
+  __shared__ double top[kClusterThreads / 32];
+  __shared__ int starts[kClusterThreads / 32], first[kN + 1];
+  const int x = threadIdx.x, lane = x & 31, warp = x >> 5;
+  const double v = x < n ? L.ev[x] : 0.0;
+  double mx = fabs(v);
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (lane == 0) top[warp] = mx;
+  __syncthreads();
+  for (int w = 0; w < kClusterThreads / 32; ++w) mx = fmax(mx, top[w]);
   const double ortol = 1e-4 * fmax(mx, 1e-300);
-  int nc = 0, start = 0;
-  for (int x = 1; x < n; ++x)
-    if (L.ev[x] - L.ev[x - 1] > ortol) {
-      L.cl_block[nc] = 0; L.cl_first[nc] = start; L.cl_count[nc] = x - start; ++nc; start = x;
-    }
-  L.cl_block[nc] = 0; L.cl_first[nc] = start; L.cl_count[nc] = n - start; ++nc;
-  for (int c = nc; c < n; ++c) { L.cl_block[c] = 0; L.cl_first[c] = 0; L.cl_count[c] = 0; }
+  const bool start = x < n && (x == 0 || v - L.ev[x - 1] > ortol);
+  const unsigned mask = __ballot_sync(0xffffffffu, start);
+  if (lane == 0) starts[warp] = __popc(mask);
+  __syncthreads();
+  int c = __popc(mask & ((1u << lane) - 1u)), nc = 0;
+  for (int w = 0; w < kClusterThreads / 32; ++w) {
+    if (w < warp) c += starts[w];
+    nc += starts[w];
+  }
+  if (start) first[c] = x;
+  if (x == 0) first[nc] = n;
+  __syncthreads();
+  if (x < n) {
+    L.cl_block[x] = 0;
+    L.cl_first[x] = x < nc ? first[x] : 0;
+    L.cl_count[x] = x < nc ? first[x + 1] - first[x] : 0;
+  }
 }
 
 }  // namespace
@@ -136,7 +155,7 @@ extern "C" nrg_status nrg_diag_block_noalloc(int n, const double* a, double* eig
   ea.flag = L.flag; ea.maxn = n; ea.rows2 = (int64_t)n * n; ea.fde = L.fde; ea.e2 = L.e2; ea.split = L.split;
   launch_bisect(ea, L.state_block, s);
   if (cudaGetLastError() != cudaSuccess) return NRG_ERR_CUDA;
-  cluster_kernel<<<1, 32, 0, s>>>(L, n);
+  cluster_kernel<<<1, kClusterThreads, 0, s>>>(L, n);
   if (cudaGetLastError() != cudaSuccess) return NRG_ERR_CUDA;
   InvIterArgs ia{};
   ia.nblocks = 1; ia.bsize = L.bsize; ia.soff = L.soff; ia.d = L.d; ia.e = L.e; ia.ev = L.ev; ia.nvec = L.nvec;
