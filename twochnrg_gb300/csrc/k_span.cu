@@ -80,7 +80,7 @@ __host__ __device__ inline size_t span_ex_doubles(int maxn, int G, int R) {
 }
 // Shared memory besides the rows.
 __host__ __device__ inline size_t span_fixed_doubles(int n, int G) {
-  return 3 * ((size_t)n + (n & 1) + kPad) + 2 * (((size_t)n + G - 1) / G) + kSweep * 32 + kSweep * kSweep + 6 + 2;
+  return 3 * ((size_t)n + (n & 1) + kPad) + 4 * (((size_t)n + G - 1) / G) + kSweep * 32 + kSweep * kSweep + 6 + 2;
 }
 
 struct SpanSm {
@@ -88,6 +88,8 @@ struct SpanSm {
   double* y;     // y of the last step
   double* tot;   // row products and next-column elements of the CTA's own rows
   double* acol;
+  double* p;     // -p_r and -q_r of the own rows
+  double* q;
   double* part;  // norm partials of the sweep threads
   double* quart; // row products of the split rows, by warp
   double* sc;    // scalars of the step
@@ -95,7 +97,7 @@ struct SpanSm {
   int ldv, ld;
 };
 
-enum { SC_BETA, SC_TU1, SC_B, SC_TAU, SC_H2 };
+enum { SC_BETA, SC_TU1, SC_B, SC_H2 };
 
 // RT of the CTA's rows at `row` (own rows i0, i0 + di, ...): the pending update
 // and the product with x over strips s0 .. s1-1 of columns j+1..n-1, whose sums
@@ -105,14 +107,11 @@ __device__ __forceinline__ void span_rows(const SpanSm& S, double* row, int64_t 
                                           int di, int s0, int s1, double* out, int od, const double* xc,
                                           const double* uo) {
   const int lane = threadIdx.x & 31, step = (int)(di * ld);
-  const double tau = S.sc[SC_TAU], h2 = S.sc[SC_H2];
   double p[RT], q[RT], acc[RT];
 #pragma unroll
   for (int k = 0; k < RT; ++k) {
-    const int r = rank + G * (i0 + k * di);
-    const double u = uo[r];
-    p[k] = -tau * u;
-    q[k] = fma(h2, u, -tau * S.y[r]);
+    p[k] = S.p[i0 + k * di];
+    q[k] = S.q[i0 + k * di];
     acc[k] = 0.0;
   }
   int c = j + 1 + 32 * s0 + lane;
@@ -243,6 +242,8 @@ __global__ void __launch_bounds__(kSpanThreads, 1) tridiag_span_kernel(TridiagAr
       S.y = p; p += S.ldv;
       S.tot = p; p += om;
       S.acol = p; p += om;
+      S.p = p; p += om;
+      S.q = p; p += om;
       S.part = p; p += kSweep * 32;
       S.quart = p; p += kSweep * kSweep;
       S.sc = p; p += 6;
@@ -263,7 +264,7 @@ __global__ void __launch_bounds__(kSpanThreads, 1) tridiag_span_kernel(TridiagAr
       S.x[S.ldv + c] = 0.0;                  // no update pending
       S.y[c] = 0.0;
     }
-    if (tid < 6) S.sc[tid] = 0.0;
+    for (int i = tid; i < own; i += kSpanThreads) S.p[i] = S.q[i] = 0.0;
     group_barrier(E, arrived += G, dead, A.flag);  // row 0 is read before it is overwritten
     if (warp < kSweep) {  // norm partials of the first x (elements 2..n-1)
       double s = 0.0;
@@ -377,7 +378,6 @@ __global__ void __launch_bounds__(kSpanThreads, 1) tridiag_span_kernel(TridiagAr
         const double t = tau * dv;  // of the block's scale, where tau^2 may leave the range
         if (lane == 0) {
           S.sc[SC_B] = fma(-tu1, t, tau * v1.x);
-          S.sc[SC_TAU] = tau;
           S.sc[SC_H2] = tau * t;
           xc[j + 1] = u1;
         }
@@ -414,6 +414,16 @@ __global__ void __launch_bounds__(kSpanThreads, 1) tridiag_span_kernel(TridiagAr
         }
       }
       __syncthreads();
+      if (warp == kSweep) {  // the own rows' part of the update, one lane each
+        const double h2 = S.sc[SC_H2];
+#pragma unroll 1
+        for (int i = i0 + lane; i < own; i += 32) {
+          const int r = rank + G * i;
+          const double u = xc[r];
+          S.p[i] = -tau * u;
+          S.q[i] = fma(h2, u, -tau * fma(-beta, S.acol[i], total(i)));
+        }
+      }
       if (warp < kSweep) {
         const double bb = S.sc[SC_B];
         double s = 0.0;
@@ -432,8 +442,7 @@ __global__ void __launch_bounds__(kSpanThreads, 1) tridiag_span_kernel(TridiagAr
     if (rank == (n - 1) % G && tid == 0) {
       const int i = (n - 1) / G;
       double a = i < ng ? gbase[i * gld + n - 1] : sbase[i * S.ld + n - 1];
-      const double u = uo[n - 1], y = S.y[n - 1], tau = S.sc[SC_TAU];
-      a = fma(-tau * u, y, fma(fma(S.sc[SC_H2], u, -tau * y), u, a));
+      a = fma(S.p[i], S.y[n - 1], fma(S.q[i], uo[n - 1], a));
       A.d[so + n - 2] = xc[n - 2];
       A.e[so + n - 2] = xc[n - 1];
       A.d[so + n - 1] = a;
