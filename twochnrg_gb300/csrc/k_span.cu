@@ -45,6 +45,7 @@ constexpr int kSweep = 4;                        // sweep warps, one per sub-par
 constexpr int kSpanThreads = (kSweep + 2) * 32;  // + the scalar warp + one that empties the exchange entries
 constexpr int kPad = 32;                         // zeros past the vectors' ends
 constexpr int kSplitCols = 128;                  // at least a strip of columns per warp
+constexpr int kPollCols = 768;                   // from here on the gather waits for the shares
 constexpr int kBufs = 3;
 constexpr long long kEmpty = -1;                 // a NaN that no FP64 operation gives
 constexpr long long kWaitCycles = 4000000000ll;  // about two seconds
@@ -180,6 +181,33 @@ __device__ __forceinline__ void span_split(const SpanSm& S, double* base, int64_
     i += 2;
   }
   if (i < end) span_rows<1>(S, base + i * ld, ld, G, rank, n, j, i, 1, s0, s1, S.quart + (i - first) * kSweep + warp, kSweep, xc, uo);
+}
+
+// The gathered y and the first part of the next x, L entries per thread in flight
+// (a round trip through L2 each).
+template <int L>
+__device__ __forceinline__ void gather(const SpanSm& S, const double2* pair, int j, int n, double tu1, double* uo,
+                                       volatile int* dead, int* flag) {
+#pragma unroll 1
+  for (int c = j + 1 + (int)threadIdx.x; c < n; c += L * kSweep * 32) {
+    double2 v[L];
+#pragma unroll
+    for (int k = 0; k < L; ++k) v[k] = load_pair(pair + min(c + k * kSweep * 32, n - 1));
+#pragma unroll
+    for (int k = 0; k < L; ++k) {
+      const int ck = c + k * kSweep * 32;
+      if (ck >= n) break;
+      if (!is_full(v[k]) && !*dead) {
+        const long long t0 = clock64();
+        do {
+          if (clock64() - t0 > kWaitCycles) { *dead = 1; atomicOr(flag, DEV_TIMEOUT); }
+          v[k] = load_pair(pair + ck);
+        } while (!is_full(v[k]) && !*dead);
+      }
+      uo[ck] = fma(-tu1, v[k].x, v[k].y);
+      S.y[ck] = v[k].x;
+    }
+  }
 }
 
 // Barrier of the group: every CTA arrives once per call.
@@ -366,6 +394,7 @@ __global__ void __launch_bounds__(kSpanThreads, 1) tridiag_span_kernel(TridiagAr
           dv += (q0 + lane < G ? va : 0.0) + (q0 + lane + 32 < G ? vb : 0.0);
         }
         __syncwarp();
+        if (m > kPollCols) asm volatile("barrier.cta.arrive 1, %0;" ::"n"((kSweep + 1) * 32) : "memory");
         dv = warp_sum_fixed(dv);
         if (!is_full(v1) && !*dead) {
           const long long t0 = clock64();
@@ -392,25 +421,16 @@ __global__ void __launch_bounds__(kSpanThreads, 1) tridiag_span_kernel(TridiagAr
         if (rank == j % G)  // u_j into row j, which no CTA reads any more (the scalar warp writes u_1)
           for (int c = j + 2 + tid; c < n; c += kSweep * 32) H[(int64_t)j * n + c] = xc[c];
         // x of the next step: column j+1 of A - p y^T - q u^T, in two parts.
-#pragma unroll 1
-        for (int c = j + 1 + tid; c < n; c += 4 * kSweep * 32) {
-          double2 v[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) v[k] = load_pair(pair + min(c + k * kSweep * 32, n - 1));
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int ck = c + k * kSweep * 32;
-            if (ck >= n) break;
-            if (!is_full(v[k]) && !*dead) {
-              const long long t0 = clock64();
-              do {
-                if (clock64() - t0 > kWaitCycles) { *dead = 1; atomicOr(A.flag, DEV_TIMEOUT); }
-                v[k] = load_pair(pair + ck);
-              } while (!is_full(v[k]) && !*dead);
-            }
-            uo[ck] = fma(-tu1, v[k].x, v[k].y);
-            S.y[ck] = v[k].x;
-          }
+        // Few entries per thread are polled as they come.  Many would crowd the L2
+        // lines that are still to be written: they are read once the scalar warp
+        // has every share, when all are there or about to be.  One block of 1901 /
+        // 1000 / 600 states: polled 2, 4, 8 deep 25.8, 26.0, 35.5 / 6.70, 6.96, 8.67
+        // / 3.03, 3.14, 3.20 ms; after the shares 8 deep 25.0 / 6.85 / 3.11 ms.
+        if (m > kPollCols) {
+          asm volatile("barrier.cta.sync 1, %0;" ::"n"((kSweep + 1) * 32) : "memory");
+          gather<8>(S, pair, j, n, tu1, uo, dead, A.flag);
+        } else {
+          gather<2>(S, pair, j, n, tu1, uo, dead, A.flag);
         }
       }
       __syncthreads();
