@@ -425,7 +425,7 @@ int cluster_threads(bool shared_gpu) {
 // Blocks up to this many states go to the row kernel (k_rows.cu), as long as
 // their rows fit in the shared memory of a cluster of 16 (617 states on a
 // GB300): 1.9 times faster than the lower-triangle cluster kernel at 600 states
-// (6.14 against 11.6 ms), 3.6 times at 256, 5.4 times at 64.
+// (6.04 against 11.6 ms), 3.7 times at 256, 5.6 times at 64.
 int rows_block_threshold() {
   const char* s = std::getenv("NRG_ROWS_N");
   return s ? std::atoi(s) : 617;

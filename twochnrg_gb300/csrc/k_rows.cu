@@ -15,6 +15,8 @@
 //  * the reflector u = x - beta e_1 stays unnormalized (H = I - tau u u^T), and
 //    A u = A x - beta (A e_1), so that the sweep starts from x while a warp of
 //    its own forms |x|, beta and tau;
+//  * the pending update is kept as A - p y^T - q u^T with p_r = tau u_r and q_r =
+//    tau y_r - 2 h u_r of the own rows, so that no w is formed over the columns;
 //  * the gather carries the column of the next step beside y, so that every
 //    CTA forms the next x for itself; it goes by st.async to the CTAs' own
 //    mbarriers (about 400 cycles), where a cluster barrier after remote stores
@@ -25,10 +27,12 @@
 // loops below have warp-uniform bounds (the vectors end in kPad zeros), are not
 // unrolled where they may end early, and compare doubles as integers.
 // One block alone (kernel with its launch, GB300): 64 / 128 / 256 / 400 / 600
-// states in 0.125 / 0.289 / 0.914 / 2.31 / 6.14 ms on 16 CTAs, where the
-// lower-triangle cluster kernel (k_tridiag.cu) took 0.674 / 1.51 / 3.25 / 6.07 /
-// 11.6 ms; the sweep's FP64 work alone is 0.8 ms of the 0.914 at 256 on the 32
-// operations per 19 cycles an SM does.
+// states in 0.119 / 0.275 / 0.878 / 2.24 / 6.04 ms on 16 CTAs (0.125 / 0.289 /
+// 0.914 / 2.31 / 6.14 with w formed over the columns), where the lower-triangle
+// cluster kernel (k_tridiag.cu) took 0.674 / 1.51 / 3.25 / 6.07 / 11.6 ms.  The
+// FP64 work of the sweep, 3 FMA per element at 1.7 per cycle and SM, is 0.33 of
+// the 0.878 ms at 256 and 4.2 of the 6.04 at 600; the rest is the chain of one
+// column, 1.9 us at any size.
 //
 // Waits: an mbarrier wait per step, bounded; cluster barriers per block.
 //
@@ -91,10 +95,10 @@ __device__ __forceinline__ bool try_wait(uint32_t bar, uint32_t parity) {
 
 struct RowsSm {
   double* x;      // 2 x ldv: u of the last step, x of this one
-  double* w;
+  double* y;      // y of the last step
   double2* ya;    // 2 x ldv: gathered (y, next column), by step parity
-  double* tot;    // row products and next-column elements of the CTA's own rows
-  double* acol;
+  double* tot;    // own rows: products, then -p_r of the update they lead to
+  double* acol;   // own rows: next-column elements, then -q_r
   double* part;   // norm partials of the sweep threads
   double* dp;     // 2 x kMaxCl partial dots
   double* sc;     // scalars of the step
@@ -104,7 +108,7 @@ struct RowsSm {
   int ldv, ld;
 };
 
-enum { SC_TAU, SC_BETA, SC_TU1, SC_B, SC_H, SC_COUNT = 6 };
+enum { SC_BETA, SC_TU1, SC_B, SC_COUNT = 4 };
 
 __host__ __device__ inline size_t rows_smem_doubles(int maxn, int cl) {
   const size_t ldv = (size_t)maxn + (maxn & 1) + kPad, own = ((size_t)maxn + cl - 1) / cl;
@@ -119,7 +123,7 @@ __device__ inline RowsSm rows_carve(double* sm, int maxn, int cl) {
   double* p = sm;
   S.ya = (double2*)p; p += 4 * S.ldv;
   S.x = p; p += 2 * S.ldv;
-  S.w = p; p += S.ldv;
+  S.y = p; p += S.ldv;
   S.tot = p; p += own;
   S.acol = p; p += own;
   S.part = p; p += kSweep * 32;
@@ -131,20 +135,19 @@ __device__ inline RowsSm rows_carve(double* sm, int maxn, int cl) {
   return S;
 }
 
-// RT of the CTA's rows: the pending rank-2 update (uo, wo) and the product
-// with x over columns j+1..n-1.
+// RT of the CTA's rows: the pending update A - p y^T - q u^T and the product with
+// x over columns j+1..n-1.
 template <int RT>
 __device__ __forceinline__ void sweep_rows(const RowsSm& S, int CL, int rank, int n, int j, int i0, const double* xc,
                                            const double* uo) {
   const int lane = threadIdx.x & 31;
   double* row = S.rows + i0 * S.ld;
   const int step = kSweep * S.ld;
-  double ur[RT], wr[RT], acc[RT];
+  double pr[RT], qr[RT], acc[RT];
 #pragma unroll
   for (int q = 0; q < RT; ++q) {
-    const int r = rank + CL * (i0 + q * kSweep);
-    ur[q] = -uo[r];
-    wr[q] = -S.w[r];
+    pr[q] = S.tot[i0 + q * kSweep];
+    qr[q] = S.acol[i0 + q * kSweep];
     acc[q] = 0.0;
   }
   const int ns = (n - j - 1 + 31) >> 5;
@@ -152,20 +155,20 @@ __device__ __forceinline__ void sweep_rows(const RowsSm& S, int CL, int rank, in
   auto col = [n](int k) { return min(k, n - 1); };  // past the row's end the vectors are 0
   // A sub-partition runs one sweep warp, so the next strip is loaded before
   // this one's FMAs (90 cycles per FMA without, 74 with; 72 is the pipe's).
-  double u = uo[c], w = S.w[c], x = xc[c], r[RT];
+  double u = uo[c], y = S.y[c], x = xc[c], r[RT];
 #pragma unroll
   for (int q = 0; q < RT; ++q) r[q] = row[q * step + col(c)];
   for (int k = 0; k < ns; ++k, c += 32) {
-    double un = 0.0, wn = 0.0, xn = 0.0, rn[RT];
+    double un = 0.0, yn = 0.0, xn = 0.0, rn[RT];
     if (k + 1 < ns) {
-      un = uo[c + 32]; wn = S.w[c + 32]; xn = xc[c + 32];
+      un = uo[c + 32]; yn = S.y[c + 32]; xn = xc[c + 32];
 #pragma unroll
       for (int q = 0; q < RT; ++q) rn[q] = row[q * step + col(c + 32)];
     }
 #pragma unroll
-    for (int q = 0; q < RT; ++q) r[q] = fma(wr[q], u, r[q]);
+    for (int q = 0; q < RT; ++q) r[q] = fma(qr[q], u, r[q]);
 #pragma unroll
-    for (int q = 0; q < RT; ++q) r[q] = fma(ur[q], w, r[q]);
+    for (int q = 0; q < RT; ++q) r[q] = fma(pr[q], y, r[q]);
 #pragma unroll
     for (int q = 0; q < RT; ++q) acc[q] = fma(r[q], x, acc[q]);
 #pragma unroll
@@ -173,7 +176,7 @@ __device__ __forceinline__ void sweep_rows(const RowsSm& S, int CL, int rank, in
       if (c < n) row[q * step + c] = r[q];
       r[q] = rn[q];
     }
-    u = un; w = wn; x = xn;
+    u = un; y = yn; x = xn;
   }
   if (lane == 0) {
 #pragma unroll
@@ -249,8 +252,9 @@ __global__ void __launch_bounds__(kRowsThreads, 3) tridiag_rows_kernel(TridiagAr
     for (int c = tid; c < n + kPad; c += kRowsThreads) {
       S.x[c] = c < n ? __ldcg(H + c) : 0.0;
       S.x[S.ldv + c] = 0.0;  // no update pending
-      S.w[c] = 0.0;
+      S.y[c] = 0.0;
     }
+    for (int i = tid; i < own; i += kRowsThreads) S.tot[i] = S.acol[i] = 0.0;
     if (tid == 0 && n > 2 && !*dead) expect_bytes(smem_u32(S.bar + (g & 1)), step_bytes(n - 1, CL));
     cluster_sync();  // every row is read before any is overwritten, every mbarrier armed
     if (warp < kSweep) {  // norm partials of the first x (elements 2..n-1)
@@ -261,7 +265,7 @@ __global__ void __launch_bounds__(kRowsThreads, 3) tridiag_rows_kernel(TridiagAr
     __syncthreads();
 
     double* xc = S.x;          // column j of A^(j); x[j] = d_j
-    double* uo = S.x + S.ldv;  // u_{j-1}, with S.w pending
+    double* uo = S.x + S.ldv;  // u_{j-1}, its update pending with S.y
     for (int j = 0; j + 2 < n; ++j, ++g) {
       const int m = n - j - 1;
       double2* ya = S.ya + (g & 1) * S.ldv;
@@ -272,7 +276,7 @@ __global__ void __launch_bounds__(kRowsThreads, 3) tridiag_rows_kernel(TridiagAr
       // reduction over the own rows before it and one over the CTAs after it).
       const bool split_dot = split_dot_at(m, CL);
       const int i0 = j + 1 <= rank ? 0 : (j + 1 - rank + CL - 1) / CL;  // first own row of the trailing matrix
-      double tau = 0.0, beta, u1, tu1 = 0.0, rs = 0.0, sum = 1.0;
+      double tau = 0.0, beta, u1, tu1 = 0.0, rs = 0.0, sum = 1.0, h2 = 0.0;
       if (warp == kSweep) {
         // The next step's mbarrier is armed before this step's stores go out, so
         // that no store for that step can come before it.
@@ -322,9 +326,6 @@ __global__ void __launch_bounds__(kRowsThreads, 3) tridiag_rows_kernel(TridiagAr
           put1(map_rank(smem_u32(dp + rank), lane), 0.0, map_rank(bar, lane));  // the token
         }
         tau = rs * fast_rcp(sum);  // 2 / u.u = 1 / (|x| (|x| + |alpha|))
-        if (lane == 0) S.sc[SC_TAU] = tau;
-        __syncwarp();
-        asm volatile("barrier.cta.arrive 1, %0;" ::"n"(kRowsThreads) : "memory");
         if (rank == j % CL) {
           if (lane == 0) { A.d[so + j] = xc[j]; A.e[so + j] = beta; A.tau[so + j] = tau; H[(int64_t)j * n + j + 1] = u1; }
         }
@@ -339,9 +340,6 @@ __global__ void __launch_bounds__(kRowsThreads, 3) tridiag_rows_kernel(TridiagAr
         }
         if (rank == j % CL)  // u_j into row j, which no CTA reads any more (the scalar warp writes u_1)
           for (int c = j + 2 + tid; c < n; c += kSweep * 32) H[(int64_t)j * n + c] = xc[c];
-        __syncwarp();
-        asm volatile("barrier.cta.sync 1, %0;" ::"n"(kRowsThreads) : "memory");
-        tau = S.sc[SC_TAU];
       }
       // Bounded.  A CTA whose wait gives up raises the flag, stops storing to
       // the others and arming its mbarriers, and runs on (its numbers void) to
@@ -369,10 +367,10 @@ __global__ void __launch_bounds__(kRowsThreads, 3) tridiag_rows_kernel(TridiagAr
         }
         dv = warp_sum_fixed(dv);
         const double t = tau * dv;  // of the block's scale, where tau^2 may leave the range
-        const double b = fma(-tu1, t, tau * ya[j + 1].x), h = 0.5 * tau * t;
+        const double b = fma(-tu1, t, tau * ya[j + 1].x);
+        h2 = tau * t;
         if (lane == 0) {
           S.sc[SC_B] = b;
-          S.sc[SC_H] = h;
           xc[j + 1] = u1;
         }
       } else {
@@ -380,30 +378,35 @@ __global__ void __launch_bounds__(kRowsThreads, 3) tridiag_rows_kernel(TridiagAr
         for (int c = j + 1 + tid; c < n; c += kSweep * 32) {
           const double2 v = ya[c];
           uo[c] = fma(-tu1, v.x, v.y);
-          S.w[c] = tau * v.x;
+          S.y[c] = v.x;
         }
       }
       __syncthreads();
       if (warp < kSweep) {
-        const double bb = S.sc[SC_B], h = S.sc[SC_H];
+        const double bb = S.sc[SC_B];
         double s = 0.0;
 #pragma unroll 1
         for (int c = j + 1 + tid; c < n; c += kSweep * 32) {
-          const double u = xc[c];
-          const double x = fma(-bb, u, uo[c]);
+          const double x = fma(-bb, xc[c], uo[c]);
           uo[c] = x;
-          S.w[c] = fma(-h, u, S.w[c]);
           s = fma(x, c >= j + 3 ? x : 0.0, s);
         }
         S.part[tid] = s;
+      } else {  // the own rows' part of the update, one lane each
+#pragma unroll 1
+        for (int i = i0 + lane; i < own; i += 32) {
+          const double u = xc[rank + CL * i], y = fma(-beta, S.acol[i], S.tot[i]);
+          S.tot[i] = -tau * u;
+          S.acol[i] = fma(h2, u, -tau * y);
+        }
       }
       __syncthreads();
       double* t = xc; xc = uo; uo = t;
     }
     // The last 2 x 2 block: row n-2 is the last x; the corner has its update pending.
     if (rank == (n - 1) % CL && tid == 0) {
-      double a = S.rows[(size_t)((n - 1) / CL) * S.ld + n - 1];
-      if (n > 2) a = fma(-uo[n - 1], S.w[n - 1], fma(-S.w[n - 1], uo[n - 1], a));
+      const int i = (n - 1) / CL;
+      const double a = fma(S.tot[i], S.y[n - 1], fma(S.acol[i], uo[n - 1], S.rows[(size_t)i * S.ld + n - 1]));
       A.d[so + n - 2] = xc[n - 2];
       A.e[so + n - 2] = xc[n - 1];
       A.d[so + n - 1] = a;
