@@ -478,6 +478,13 @@ int grid_split(int nbig) {
   return std::min(k, nbig);
 }
 
+// The stream for what runs beside the context's own, with its fork and join events.
+void ensure_second_stream(nrg_ctx* c) {
+  if (!c->rows_stream) CU(cudaStreamCreateWithFlags(&c->rows_stream, cudaStreamNonBlocking));
+  if (!c->rows_fork) CU(cudaEventCreateWithFlags(&c->rows_fork, cudaEventDisableTiming));
+  if (!c->rows_join) CU(cudaEventCreateWithFlags(&c->rows_join, cudaEventDisableTiming));
+}
+
 // Cooperative grids of different contexts (the chain sweep beside the
 // impurity sweep, batch workers) never run at the same time: the grids of one
 // context together ask for one CTA per SM, and two contexts' grids, each
@@ -861,11 +868,7 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
     h2d(c, c->rlist.p, pk.host.data(), pk.host.size());
   }
   if (both) {
-    if (!c->rows_stream) {
-      CU(cudaStreamCreateWithFlags(&c->rows_stream, cudaStreamNonBlocking));
-      CU(cudaEventCreateWithFlags(&c->rows_fork, cudaEventDisableTiming));
-      CU(cudaEventCreateWithFlags(&c->rows_join, cudaEventDisableTiming));
-    }
+    ensure_second_stream(c);
     CU(cudaEventRecord(c->rows_fork, c->stream));
     CU(cudaStreamWaitEvent(c->rows_stream, c->rows_fork, 0));
   }
@@ -978,7 +981,13 @@ void run_vectors(nrg_ctx* c, Timer& tm, EigPlan& P, const std::vector<double>& e
   const int gsplit = gmaxn >= 300 && 2 * glen <= 4 * (int64_t)c->num_sms * gmaxn ? 2 : 1;
   const int gw = gsplit > 1 ? 2 : gvecs < 8 * c->num_sms ? 4 : 8;
   const int bw = backtransform_warps(lmaxn);
-  for (int b = 0; b < nb; ++b) {
+  // The largest blocks first: a vector's time goes with its block's size (inverse
+  // iteration) or the square (back-transformation, 21 ms for a CTA at 4341 states),
+  // and the kernels end with their last CTA.
+  std::vector<int> by_size(nb);
+  for (int b = 0; b < nb; ++b) by_size[b] = b;
+  std::stable_sort(by_size.begin(), by_size.end(), [&](int x, int z) { return P.bsize[x] > P.bsize[z]; });
+  for (int b : by_size) {
     const int n = P.bsize[b], k = P.nvec[b];
     if (k == 0) continue;
     double onenrm = 0.0;
@@ -1028,6 +1037,16 @@ void run_vectors(nrg_ctx* c, Timer& tm, EigPlan& P, const std::vector<double>& e
   ba.nvec = ia.nvec; ba.yoff = ia.yoff; ba.Y = c->Y.as<double>(); ba.Z = c->Z.as<double>(); ba.Zt = c->Zt.as<double>();
   ba.zoff = ia.yoff; ba.maxn = lmaxn;
   cudaEvent_t t1 = tm.start();
+  // Both kinds of blocks at once: the grouped CTAs fill the SMs that the long ones
+  // leave.
+  const bool both = !ctab.empty() && !gtab.empty();
+  cudaStream_t gs = c->stream;
+  if (both) {
+    ensure_second_stream(c);
+    gs = c->rows_stream;
+    CU(cudaEventRecord(c->rows_fork, c->stream));
+    CU(cudaStreamWaitEvent(gs, c->rows_fork, 0));
+  }
   if (!ctab.empty()) {
     CU(launch_backtransform(ba, (const int*)(base + o_tb), (const int*)(base + o_tf), (int)ctab.size(), c->stream));
     c->launches++;
@@ -1036,10 +1055,14 @@ void run_vectors(nrg_ctx* c, Timer& tm, EigPlan& P, const std::vector<double>& e
     ba.maxn = gmaxn;
     ba.grp_block = (const int*)(base + o_pb); ba.grp_index = (const int*)(base + o_pi);
     ba.grp_first = (const int*)(base + o_pf); ba.factors = c->bfac.as<double>();
-    launch_back_factors(ba, (int)grpb.size(), c->stream);
+    launch_back_factors(ba, (int)grpb.size(), gs);
     CU(launch_backtransform_grouped(ba, (const int*)(base + o_gb), (const int*)(base + o_gf), (int)gtab.size(), gw,
-                                    gsplit, c->stream));
+                                    gsplit, gs));
     c->launches += 2;
+  }
+  if (both) {
+    CU(cudaEventRecord(c->rows_join, gs));
+    CU(cudaStreamWaitEvent(c->stream, c->rows_join, 0));
   }
   tm.stop(t1, &c->timing.backtransform_ms);
   double fl = 0.0;
@@ -1222,16 +1245,16 @@ AsmTables prepare_assembly(nrg_ctx* c, const ModelSpec& m, const Basis& B, const
   return T;
 }
 
-// One matrix of a grouped GEMM launch: its index in the launch's list, rows and
-// columns.
-struct TileDim { int id, m, n; };
+// One matrix of a grouped GEMM launch: its index in the launch's list, rows,
+// columns and length of its sums.
+struct TileDim { int id, m, n, k; };
 
 // The matrices cut into tiles of 4 R rows x kGemmTile columns, listed by matrix in
 // (id, mn); returns R.  A tile takes R units of time (gemm_tile.cuh) and an SM one
 // tile at a time, whichever others are resident: the R with the fewest units, the
 // largest of equal ones (fewer loads).  The list is run `times` times in one launch.  Tangent sweep at 200 kept, 10 to 60 tiles
 // of 32 rows per launch: 50 ms with tiles of 32 rows only, 40.5 ms so.
-int cut_tiles(const std::vector<TileDim>& dims, int sms, int times, std::vector<int>& id, std::vector<int>& mn) {
+int cut_tiles(std::vector<TileDim>& dims, int sms, int times, std::vector<int>& id, std::vector<int>& mn) {
   int best = 8;
   int64_t least = std::numeric_limits<int64_t>::max();
   for (int R = 8; R >= 2; R /= 2) {
@@ -1240,6 +1263,8 @@ int cut_tiles(const std::vector<TileDim>& dims, int sms, int times, std::vector<
     const int64_t units = (tiles * times + sms - 1) / sms * R;
     if (units < least) { least = units; best = R; }
   }
+  // the longest sums first: a launch ends with its last tile
+  std::stable_sort(dims.begin(), dims.end(), [](const TileDim& a, const TileDim& b) { return a.k > b.k; });
   for (const TileDim& d : dims)
     for (int mt = 0; mt * 4 * best < d.m; ++mt)
       for (int nt = 0; nt * kGemmTile < d.n; ++nt) { id.push_back(d.id); mn.push_back((mt << 16) | nt); }
@@ -1357,10 +1382,10 @@ void plan_update(UpdatePlan& U, int sms, int ndir, const ModelSpec& m, const Bas
             if ((int)U.terms1.size() > first1) {
               const int gid = (int)U.g1first.size();
               U.g1first.push_back(first1); U.g1count.push_back((int)U.terms1.size() - first1);
-              dims1.push_back({gid, p.count, J.kj});
+              dims1.push_back({gid, p.count, J.kj, 0});
             }
           }
-        dims.push_back({jid, J.ki, J.kj});
+        dims.push_back({jid, J.ki, J.kj, J.nI});
       }
   }
   U.rows = cut_tiles(dims, sms, ndir, U.tjob, U.tmn);
@@ -1437,7 +1462,7 @@ struct GemmPlan {
 void run_gemm_plan(nrg_ctx* c, const GemmPlan& G) {
   if (G.jobs.empty()) return;
   std::vector<TileDim> dims;
-  for (size_t k = 0; k < G.jobs.size(); ++k) dims.push_back({(int)k, G.jobs[k].m, G.jobs[k].n});
+  for (size_t k = 0; k < G.jobs.size(); ++k) dims.push_back({(int)k, G.jobs[k].m, G.jobs[k].n, G.jobs[k].k});
   std::vector<int> tjob, tmn;
   const int rows = cut_tiles(dims, c->num_sms, 1, tjob, tmn);
   Packer pk;
