@@ -686,15 +686,18 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
   // beside the row kernel, split where the sum of both is smallest: 2600 states
   // 74 ms by the span kernel, 84 by the grid; 3400 states 160 and 138; two / three
   // blocks of 1900 52 / 70 ms and 56 / 64; eight of 1200 42 ms (cluster kernel 86).
+  // The mixed form keeps its large blocks and has the others after them too: beside
+  // the panels, which are launched again and again, they took the SMs that the next
+  // panel waited for (0.96 s a full-size iteration, 0.64 so).
   SpanPlan sp;
   const bool cluster_only = std::getenv("NRG_CLUSTER") || std::getenv("NRG_CLUSTER_THREADS");
-  if (!c->shared_gpu && !cluster_only && !(mixed && nbig > 0) && nb > 0 && P.bsize[order_h[0]] > span_from()) {
+  if (!c->shared_gpu && !cluster_only && nb > 0 && P.bsize[order_h[0]] > span_from()) {
     std::vector<int> sizes(nb);
     int must = 0;
     for (int q = 0; q < nb; ++q) sizes[q] = P.bsize[order_h[q]];
     while (must < nb && sizes[must] > std::max(2, rows_block_threshold())) ++must;
     const int rmax = tridiag_span_max_ctas(16) / 16;
-    const bool forced = std::getenv("NRG_BIG_N") != nullptr;  // nbig stays
+    const bool forced = (mixed && nbig > 0) || std::getenv("NRG_BIG_N") != nullptr;  // nbig stays
     double best = 1e300;
     const int k0 = forced ? nbig : 0;
     int pick = nbig;
