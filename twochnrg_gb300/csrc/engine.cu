@@ -696,7 +696,7 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
     int must = 0;
     for (int q = 0; q < nb; ++q) sizes[q] = P.bsize[order_h[q]];
     while (must < nb && sizes[must] > std::max(2, rows_block_threshold())) ++must;
-    const int rmax = tridiag_span_max_ctas(16) / 16;
+    const int rmax = tridiag_rows_max_clusters(16, 600);  // one CTA per SM
     const bool forced = (mixed && nbig > 0) || std::getenv("NRG_BIG_N") != nullptr;  // nbig stays
     double best = 1e300;
     const int k0 = forced ? nbig : 0;

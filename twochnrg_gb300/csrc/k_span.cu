@@ -479,32 +479,8 @@ __global__ void __launch_bounds__(kSpanThreads, 1) tridiag_span_kernel(TridiagAr
   }
 }
 
-// Groups of a multiple of 16 CTAs go as clusters, which keeps each one's SMs
-// together and so leaves room for the row kernel's clusters beside it.
-cudaLaunchConfig_t span_config(int ctas, bool clusters, size_t smem, cudaLaunchAttribute* attr) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)ctas, 1, 1);
-  cfg.blockDim = dim3(kSpanThreads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (clusters) {
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = 16;
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = 1;
-    cfg.numAttrs = 2;
-  }
-  return cfg;
-}
-
 cudaError_t span_attributes() {
-  cudaError_t err =
-      cudaFuncSetAttribute(tridiag_span_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem() - 1024);
-  if (err == cudaSuccess) err = cudaFuncSetAttribute(tridiag_span_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  return err;
+  return cudaFuncSetAttribute(tridiag_span_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem() - 1024);
 }
 
 // Room for the rows of the largest block, as far as there is any.
@@ -519,27 +495,22 @@ size_t tridiag_span_work(int maxn, int groups, int G, int copies) { return group
 
 bool tridiag_span_fits(int n) { return sizeof(double) * span_fixed_doubles(n, 16) <= (size_t)max_dyn_smem() - 1024; }
 
-int tridiag_span_max_ctas(int maxn) {
-  if (!tridiag_span_fits(maxn)) return 0;
-  if (span_attributes() != cudaSuccess) return 0;
-  cudaLaunchAttribute attr[2];
-  cudaLaunchConfig_t cfg = span_config(16, true, (size_t)max_dyn_smem() - 1024, attr);
-  cfg.attrs = attr + 1;
-  cfg.numAttrs = 1;
-  int nc = 0;
-  if (cudaOccupancyMaxActiveClusters(&nc, tridiag_span_kernel, &cfg) != cudaSuccess) return 0;
-  return 16 * nc;
-}
-
 cudaError_t launch_tridiag_span(const TridiagArgs& a, SpanArgs p, int groups, cudaStream_t s) {
   if (p.G < 1 || groups < 1 || p.copies < 1 || p.copies > 32) return cudaErrorInvalidValue;
   cudaError_t err = span_attributes();
   if (err != cudaSuccess) return err;
   const size_t smem = span_smem_bytes(a.maxn, p.G);
   p.smem_doubles = (int)(smem / sizeof(double));
-  cudaLaunchAttribute attr[2];
-  cudaLaunchConfig_t cfg = span_config(p.G * groups, p.clusters, smem, attr);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(p.G * groups), 1, 1);
+  cfg.blockDim = dim3(kSpanThreads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, tridiag_span_kernel, a, p);
 }
 

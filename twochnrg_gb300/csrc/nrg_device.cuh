@@ -220,19 +220,17 @@ int tridiag_max_clusters(int cluster, int maxn, int threads = 512);
 // Blocks whose rows fit in a cluster's shared memory (k_rows.cu).
 // One block per group of G CTAs, the groups' blocks in list[first[g]] ..
 // list[first[g + 1]) (k_span.cu).  A cooperative launch; work:
-// tridiag_span_work(maxn, groups, G) doubles.
+// tridiag_span_work(maxn, groups, G, copies) doubles.
 struct SpanArgs {
   const int* list;
   const int* first;
   double* work;
   int G;
   int copies;        // of the exchange area, each read by every copies-th CTA (up to 32)
-  bool clusters;     // launch as clusters of 16 (G a multiple of 16)
   int smem_doubles;  // set by the launch
 };
 size_t tridiag_span_work(int maxn, int groups, int G, int copies);
 bool tridiag_span_fits(int n);        // its vectors fit in shared memory
-int tridiag_span_max_ctas(int maxn);  // that can be resident in clusters of 16; 0: does not fit
 cudaError_t launch_tridiag_span(const TridiagArgs& a, SpanArgs p, int groups, cudaStream_t s);
 size_t tridiag_rows_smem_bytes(int maxn, int cluster);
 int tridiag_rows_max_clusters(int cluster, int maxn);
