@@ -25,7 +25,8 @@
 // per element at 1.7 per cycle and SM.  One block (kernel with its launch): 640
 // states in 8.8 / 5.2 / 3.6 / 3.5 ms on 16 / 32 / 96 / 152 CTAs, by the cluster
 // kernel of k_tridiag.cu 12.9; 1300 states in 14 ms on 152 CTAs; 1901 states in 26.7
-// ms (27.7 us per column before, now 14), by tridiag_grid_kernel 52.7.
+// ms, 24.9 with the gather as it is now (13 us per column), by tridiag_grid_kernel
+// 52.7 (27.7).
 //
 // Waits: a poll per entry and share, bounded by the clock; every CTA runs before
 // the first one (a barrier of the cooperative grid).
@@ -67,6 +68,8 @@ __device__ __forceinline__ void store_share(double* p, double v) {
   asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
 __device__ __forceinline__ bool is_full(double v) { return __double_as_longlong(v) != kEmpty; }
+// What is sent never looks empty, whatever NaN came in with the block.
+__device__ __forceinline__ double filled(double v) { return is_full(v) ? v : __longlong_as_double(0x7ff8000000000000ll); }
 __device__ __forceinline__ bool is_full(double2 v) { return is_full(v.x) && is_full(v.y); }
 
 // A group's exchange area in global memory.
@@ -415,7 +418,7 @@ __global__ void __launch_bounds__(kSpanThreads, 1) tridiag_span_kernel(TridiagAr
         tu1 = S.sc[SC_TU1];
 #pragma unroll 1
         for (int i = i0 + lane; i < own; i += 32) {
-          const double a = S.acol[i], y = fma(-beta, a, total(i));
+          const double a = filled(S.acol[i]), y = filled(fma(-beta, a, total(i)));
           for (int k = warp; k < R; k += kSweep) store_pair(pair0 + (size_t)k * kBufs * A.maxn + rank + G * i, y, a);
         }
         if (rank == j % G)  // u_j into row j, which no CTA reads any more (the scalar warp writes u_1)
