@@ -719,7 +719,7 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
   const int K = nbig > 0 ? grid_split(nbig) : 0;
   std::vector<std::vector<int>> bins(std::max(K, 1));
   size_t o_bins[nrg_ctx::kMaxSplit] = {};
-  if (K > 1) {  // deal the large blocks by cost and upload the lists before the fork
+  if (K > 1 && !mixed) {  // deal the large blocks by cost and upload the lists before the fork
     // the lower-triangle grid kernel: 2/3 n^3 FMA plus ~21 us of barriers and
     // vector work per column (2.8e6 FMA of a quarter of the GPU)
     std::vector<int> big(order_h.begin(), order_h.begin() + nbig);
@@ -785,8 +785,8 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
       for (int q = 0; q < nbig; ++q) cst[q] = cost(P.bsize[big[q]]);
       bins = deal_by_cost(big, cst, K);
     }
-    if (!c->fork) CU(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
-    CU(cudaEventRecord(c->fork, c->stream));
+    // The FP64 lists go up before the fork, which is all that the side streams'
+    // grids wait for.
     Packer pk;
     std::vector<std::vector<int>> fp(K), bl(K);
     size_t o_fp[nrg_ctx::kMaxSplit] = {};
@@ -796,6 +796,8 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
     }
     c->gbig.ensure(pk.host.size() + 256);
     h2d(c, c->gbig.p, pk.host.data(), pk.host.size());
+    if (!c->fork) CU(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
+    CU(cudaEventRecord(c->fork, c->stream));
     for (int k = 0; k < K; ++k) {
       cudaStream_t sk = c->stream;
       if (K > 1) {
