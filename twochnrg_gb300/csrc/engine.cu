@@ -1033,7 +1033,6 @@ void run_vectors(nrg_ctx* c, Timer& tm, EigPlan& P, const std::vector<double>& e
   ia.Y = c->Y.as<double>(); ia.scratch = c->scratch.as<double>();
   ia.cl_block = (const int*)(base + o_cb); ia.cl_first = (const int*)(base + o_cf); ia.cl_count = (const int*)(base + o_cn);
   ia.nclusters = (int)cb.size(); ia.flag = c->flag.as<int>();
-  ia.fde = c->fde.as<float>(); ia.nstates = P.nstates;
   cudaEvent_t t0 = tm.start();
   launch_inviter(ia, (const int*)(base + o_vb), (const int*)(base + o_vi), (int)vb.size(), c->stream);
   c->launches += 2;

@@ -160,7 +160,7 @@ extern "C" nrg_status nrg_diag_block_noalloc(int n, const double* a, double* eig
   InvIterArgs ia{};
   ia.nblocks = 1; ia.bsize = L.bsize; ia.soff = L.soff; ia.d = L.d; ia.e = L.e; ia.ev = L.ev; ia.nvec = L.nvec;
   ia.yoff = L.yoff; ia.Y = L.Y; ia.scratch = L.LU; ia.cl_block = L.cl_block; ia.cl_first = L.cl_first;
-  ia.cl_count = L.cl_count; ia.nclusters = n; ia.flag = L.flag; ia.fde = L.fde; ia.nstates = n;
+  ia.cl_count = L.cl_count; ia.nclusters = n; ia.flag = L.flag;
   launch_inviter(ia, L.vec_block, L.vec_index, n, s);
   if (cudaGetLastError() != cudaSuccess) return NRG_ERR_CUDA;
   BackArgs ba{};

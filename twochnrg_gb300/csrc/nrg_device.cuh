@@ -277,8 +277,6 @@ struct InvIterArgs {
   const int* cl_count;    // eigenvalues in the cluster
   int nclusters;
   int* flag;
-  const float* fde;       // [2*nstates] FP32 copies of d and e (launch_bisect)
-  int nstates;
 };
 void launch_inviter(const InvIterArgs& a, const int* vec_block, const int* vec_index, int nvecs,
                     cudaStream_t s);
