@@ -2620,6 +2620,7 @@ void lehmann_impl(nrg_ctx* c, const nrg_dm_params* prm, int nomega, const double
         tlo = std::max(tlo, -top);
         thi = std::min(thi, top);
       }
+      tlo = std::floor(tlo / kFgtBin) * kFgtBin;
       const double bins = std::ceil((thi - tlo) / kFgtBin);
       if (li.nrec >= fgt_min_records() && li.nrec < (int64_t)INT32_MAX && bins >= 1.0 && bins <= kFgtMaxBins) {
         FgtList f{};

@@ -610,7 +610,7 @@ struct LehmannArgs {      // A(omega) = sum_N sum_records w exp(-(t - key)^2) / 
 };
 // A list of records summed through moments of bins of its keys (k_fgt.cu).
 constexpr int kFgtMaxBins = 1024;
-constexpr int kFgtTerms = 24;
+constexpr int kFgtTerms = 28;
 constexpr double kFgtBin = 0.125;    // width of a bin in the key
 constexpr double kFgtReach = 27.5;   // exp(-x^2) is 0 beyond
 struct FgtList {
@@ -620,7 +620,7 @@ struct FgtList {
   const double* tg;
   int64_t tstride;
   int64_t nrec;
-  double origin;          // key at the first bin's lower edge
+  double origin;          // key at the first bin's lower edge, a multiple of kFgtBin
   int nbins, bin0;        // bins; first of the list's in the launch
   int chunk, nchunks, chunk0;  // records per chunk (a multiple of 256)
   int* counts;            // [nchunks][nbins]
