@@ -180,7 +180,7 @@ struct nrg_ctx {
   std::vector<double> opavg_m1;
   nrg_timing timing{};
   // device buffers
-  nrg::DevBuf meta, vmeta, H, d, e, tau, ev, en, flag, scal, Y, scratch, Z, Zt, T, partial, red, gpart, fde, e2, spl;
+  nrg::DevBuf meta, vmeta, H, d, e, tau, ev, en, flag, scal, Y, scratch, Z, Zt, T, partial, red, gpart, fde, e2, spl, rowsum;
   nrg::DevBuf ops_a[6], ops_b[6], opptr;
   nrg::DevBuf dmcnt, dmrec, dmtab;     // Lehmann record counts / offsets, records, frequency tables
   nrg::DevBuf dmtmeta;                 // work items of the tangent Lehmann sums
@@ -941,6 +941,8 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
   ea.e2 = c->e2.as<double>();
   c->spl.ensure(std::max(P.nstates, 1));
   ea.split = c->spl.as<unsigned char>();
+  c->rowsum.ensure(sizeof(double) * std::max(P.nstates, 1));
+  ea.rowsum = c->rowsum.as<double>();
   ea.mixed_n = mixed ? std::max(thr, mixed_block_threshold()) : 0;
   cudaEvent_t t1 = tm.start();
   for (int n : P.bsize) ea.rows2 += (int64_t)n * n;
@@ -1032,7 +1034,7 @@ void run_vectors(nrg_ctx* c, Timer& tm, EigPlan& P, const std::vector<double>& e
   ia.ev = c->ev.as<double>(); ia.nvec = (const int*)(base + o_nvec); ia.yoff = (const int64_t*)(base + o_yoff);
   ia.Y = c->Y.as<double>(); ia.scratch = c->scratch.as<double>();
   ia.cl_block = (const int*)(base + o_cb); ia.cl_first = (const int*)(base + o_cf); ia.cl_count = (const int*)(base + o_cn);
-  ia.nclusters = (int)cb.size(); ia.flag = c->flag.as<int>();
+  ia.nclusters = (int)cb.size(); ia.flag = c->flag.as<int>(); ia.rowsum = c->rowsum.as<double>();
   cudaEvent_t t0 = tm.start();
   launch_inviter(ia, (const int*)(base + o_vb), (const int*)(base + o_vi), (int)vb.size(), c->stream);
   c->launches += 2;

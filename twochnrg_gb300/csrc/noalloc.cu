@@ -30,13 +30,13 @@ namespace {
 
 constexpr int kN = NRG_NOALLOC_MAX_N;
 // doubles: A copy, Y, five LU arrays, d/e/tau/ev, FP32 copies of d and e
-// (2 kN floats), e^2, the split flags (kN bytes), then an integer area and the
+// (2 kN floats), e^2, the rows' 1-norms, the split flags (kN bytes), then an integer area and the
 // back-transformation's factors
 constexpr size_t kOffA = 0;
 constexpr size_t kOffY = (size_t)kN * kN;
 constexpr size_t kOffLU = 2 * (size_t)kN * kN;
 constexpr size_t kOffVec = 7 * (size_t)kN * kN;
-constexpr size_t kOffInt = kOffVec + 6 * (size_t)kN + (size_t)kN / 8 + 1;
+constexpr size_t kOffInt = kOffVec + 7 * (size_t)kN + (size_t)kN / 8 + 1;
 constexpr size_t kIntWords = 16 + 9 * (size_t)kN;  // in 4-byte words
 constexpr size_t kOffFac = kOffInt + (kIntWords + 1) / 2 + 8;
 constexpr size_t kScratchDoubles = kOffFac + 4 * (size_t)kN;  // 16 factors per group of four reflectors
@@ -46,7 +46,7 @@ static __device__ __align__(256) double g_noalloc_scratch[kScratchDoubles];
 struct Layout {
   double *A, *Y, *LU, *d, *e, *tau, *ev;
   float* fde;
-  double* e2;
+  double *e2, *rowsum;
   unsigned char* split;
   int *queue, *flag, *bsize, *soff, *order, *nvec;
   int64_t *hoff, *yoff;
@@ -60,7 +60,8 @@ Layout layout(double* base) {
   L.d = base + kOffVec; L.e = L.d + kN; L.tau = L.e + kN; L.ev = L.tau + kN;
   L.fde = reinterpret_cast<float*>(L.ev + kN);
   L.e2 = L.ev + 2 * kN;
-  L.split = reinterpret_cast<unsigned char*>(L.e2 + kN);
+  L.rowsum = L.e2 + kN;
+  L.split = reinterpret_cast<unsigned char*>(L.rowsum + kN);
   int* ip = reinterpret_cast<int*>(base + kOffInt);
   L.queue = ip; L.flag = ip + 1; L.bsize = ip + 2; L.soff = ip + 3; L.order = ip + 4; L.nvec = ip + 5;
   L.hoff = reinterpret_cast<int64_t*>(ip + 8); L.yoff = L.hoff + 1;
@@ -152,7 +153,7 @@ extern "C" nrg_status nrg_diag_block_noalloc(int n, const double* a, double* eig
   if (launch_tridiag_rows(ta, cl, 1, s) != cudaSuccess) return NRG_ERR_CUDA;
   TdEigArgs ea{};
   ea.nblocks = 1; ea.bsize = L.bsize; ea.soff = L.soff; ea.d = L.d; ea.e = L.e; ea.ev = L.ev; ea.nstates = n;
-  ea.flag = L.flag; ea.maxn = n; ea.rows2 = (int64_t)n * n; ea.fde = L.fde; ea.e2 = L.e2; ea.split = L.split;
+  ea.flag = L.flag; ea.maxn = n; ea.rows2 = (int64_t)n * n; ea.fde = L.fde; ea.e2 = L.e2; ea.split = L.split; ea.rowsum = L.rowsum;
   launch_bisect(ea, L.state_block, s);
   if (cudaGetLastError() != cudaSuccess) return NRG_ERR_CUDA;
   cluster_kernel<<<1, kClusterThreads, 0, s>>>(L, n);
@@ -160,7 +161,7 @@ extern "C" nrg_status nrg_diag_block_noalloc(int n, const double* a, double* eig
   InvIterArgs ia{};
   ia.nblocks = 1; ia.bsize = L.bsize; ia.soff = L.soff; ia.d = L.d; ia.e = L.e; ia.ev = L.ev; ia.nvec = L.nvec;
   ia.yoff = L.yoff; ia.Y = L.Y; ia.scratch = L.LU; ia.cl_block = L.cl_block; ia.cl_first = L.cl_first;
-  ia.cl_count = L.cl_count; ia.nclusters = n; ia.flag = L.flag;
+  ia.cl_count = L.cl_count; ia.nclusters = n; ia.flag = L.flag; ia.rowsum = L.rowsum;
   launch_inviter(ia, L.vec_block, L.vec_index, n, s);
   if (cudaGetLastError() != cudaSuccess) return NRG_ERR_CUDA;
   BackArgs ba{};

@@ -256,6 +256,7 @@ struct TdEigArgs {
   float* fde;            // scratch [2*nstates]: FP32 copies of d and e for the FP32 bracket
   double* e2;            // scratch [nstates]: e^2
   unsigned char* split;  // scratch [nstates]: e_i negligible (the pieces' ends)
+  double* rowsum;        // out [nstates]: 1-norms of T's rows
   int mixed_n;           // blocks of at least this many states were reduced in mixed
                          // precision (their levels carry its ~2^-36 error); <= 0: none
 };
@@ -277,6 +278,7 @@ struct InvIterArgs {
   const int* cl_count;    // eigenvalues in the cluster
   int nclusters;
   int* flag;
+  const double* rowsum;   // [nstates] of launch_bisect
 };
 void launch_inviter(const InvIterArgs& a, const int* vec_block, const int* vec_index, int nvecs,
                     cudaStream_t s);
