@@ -2473,8 +2473,9 @@ void lehmann_impl(nrg_ctx* c, const nrg_dm_params* prm, int nomega, const double
     std::vector<int> nk(s.bsize.size(), 0), nd(s.bsize.size(), 0);
     for (size_t b = 0; b < s.bsize.size(); ++b)
       for (int i = 0; i < s.bsize[b]; ++i) (s.kept[s.boff[b] + i] ? nk[b] : nd[b])++;
-    double emax = 0.0;
-    for (double e : s.en) emax = std::max(emax, e);
+    // the largest |dE|; a loaded shell's energies may start anywhere
+    double emax = s.en.empty() ? 0.0 : s.en[0], emin = emax;
+    for (double e : s.en) { emax = std::max(emax, e); emin = std::min(emin, e); }
     int64_t pbytes = 0;
     for (size_t k = 0; k < s.cd.bi.size(); ++k) pbytes += (int64_t)s.bsize[s.cd.bi[k]] * s.bsize[s.cd.bj[k]];
     c->Y.ensure(sizeof(double) * std::max<int64_t>(2 * pbytes, 1));
@@ -2618,7 +2619,7 @@ void lehmann_impl(nrg_ctx* c, const nrg_dm_params* prm, int nomega, const double
       tlo -= kFgtReach;
       thi += kFgtReach;
       if (li.gauss) {
-        const double top = std::min(a.gauss_below, emax) * a.inv_bt + kFgtBin;
+        const double top = std::min(a.gauss_below, emax - emin) * a.inv_bt + kFgtBin;
         tlo = std::max(tlo, -top);
         thi = std::min(thi, top);
       }
