@@ -35,9 +35,14 @@ constexpr int kTerms = kFgtTerms;
 constexpr double kR = 1.0 / 16;
 constexpr int kWarps = 8;
 
-__device__ __forceinline__ int bin_of(const FgtList& L, double key) {
-  const int b = (int)floor((key - L.origin) * (1.0 / (2.0 * kR)));
-  return b >= 0 && b < L.nbins ? b : -1;  // -1: its term is 0 at every frequency of the list
+__device__ __forceinline__ bool is_finite(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
+
+// -1: the record's term is 0 at every frequency of the list.  A weight that is
+// not finite makes its term NaN there too, so it is put into a bin.
+__device__ __forceinline__ int bin_of(const FgtList& L, int64_t i) {
+  const double q = floor((L.key[i] - L.origin) * (1.0 / (2.0 * kR)));
+  if (q >= 0.0 && q < (double)L.nbins) return (int)q;
+  return is_finite(L.w[i]) ? -1 : 0;
 }
 
 // Records of chunk c of the list: [begin, end); warp w of the CTA takes a
@@ -57,7 +62,7 @@ __global__ void __launch_bounds__(kWarps * 32) fgt_count_kernel(const FgtList* l
   int64_t r0, r1;
   chunk_range(L, (int)blockIdx.x - L.chunk0, &r0, &r1);
   for (int64_t i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
-    const int b = bin_of(L, L.key[i]);
+    const int b = bin_of(L, i);
     if (b >= 0) atomicAdd(&hist[b], 1);
   }
   __syncthreads();
@@ -103,7 +108,7 @@ __global__ void __launch_bounds__(kWarps * 32) fgt_sort_kernel(const FgtList* li
   for (int b = lane; b < L.nbins; b += 32) pos[warp][b] = 0;
   __syncwarp();
   for (int64_t i = w0 + lane; i < w1; i += 32) {
-    const int b = bin_of(L, L.key[i]);
+    const int b = bin_of(L, i);
     if (b >= 0) atomicAdd(&pos[warp][b], 1);
   }
   __syncthreads();
@@ -118,7 +123,7 @@ __global__ void __launch_bounds__(kWarps * 32) fgt_sort_kernel(const FgtList* li
   __syncthreads();
   for (int64_t i0 = w0; i0 < w1; i0 += 32) {
     const int64_t i = i0 + lane;
-    const int b = i < w1 ? bin_of(L, L.key[i]) : -1;
+    const int b = i < w1 ? bin_of(L, i) : -1;
     const unsigned same = __match_any_sync(0xffffffffu, b);
     const int rank = __popc(same & ((1u << lane) - 1u));
     int at = 0;
@@ -194,7 +199,10 @@ __global__ void __launch_bounds__(kWarps * 32) fgt_eval_kernel(LehmannArgs A, co
     if (L.start[b] == L.start[b + 1]) continue;
     const double centre = L.origin + (2 * b + 1) * kR;  // exact: the origin is a multiple of 2 r
     const double tau = t - centre;
-    if (fabs(tau) > 27.4) continue;  // exp(-(|tau| - r)^2) is 0
+    if (fabs(tau) > 27.4) {  // exp(-(|tau| - r)^2) is 0, and so is the term of a finite weight
+      if (!is_finite(M0[b])) acc = __longlong_as_double(0x7ff8000000000000ll);
+      continue;
+    }
     const double back = tau - t, err = (t - (tau - back)) - (centre + back);  // t - centre = tau + err
     const double sq = tau * tau, g = exp(-sq);
     double bm = 0.0, bn = fma(-g, fma(2.0 * tau, err, fma(tau, tau, -sq)), g), sum = 0.0;
