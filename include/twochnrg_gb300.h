@@ -113,7 +113,8 @@ typedef struct {
   const double* opavg;     /* [nops] CalcOpAvg of the averaged operators at betabar */
   const double* params;    /* [4] ParamsHN used: Lambda, chi_1, chi_2 (0 if 1ch; Delta_N for
                               NRG_MODEL_1CH_S), eN */
-  double wall_ms;          /* host wall time of the iteration (table building, copies, kernels) */
+  double wall_ms;          /* host wall time since the iteration before was finished (an iteration's last
+                              results are read with the next one's first) */
   double device_ms;        /* CUDA-event span of the iteration on the engine stream */
 } nrg_iteration;
 

@@ -541,7 +541,7 @@ class Iteration:
     thermo: np.ndarray
     opavg: np.ndarray
     kept_bsize: np.ndarray
-    wall_ms: float = 0.0     # host wall time of the iteration
+    wall_ms: float = 0.0     # host wall time since the iteration before was finished
     device_ms: float = 0.0   # CUDA-event span of the iteration on the engine stream
 
 

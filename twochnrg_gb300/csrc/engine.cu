@@ -1702,8 +1702,10 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
   for (int k = 0; k < 2; ++k) { CU(cudaEventCreate(&it0[k])); CU(cudaEventCreate(&it1[k])); }
   EvGuard itg0{it0[0], it1[0]}, itg1{it0[1], it1[1]};
   // What of an iteration is read when the stream is next waited for: the operator
-  // averages, its times (the host's: since the iteration before was finished).
-  c->pin_avg.ensure(sizeof(double) * 16);
+  // averages, the error flag as it stood then, its times (the host's: since the
+  // iteration before was finished).
+  constexpr int kAvg = 9;  // averages and norm, flag
+  c->pin_avg.ensure(sizeof(double) * 2 * kAvg);
   int last_N = -1;
   size_t last_avg = 0;
   auto t_last = clock::now();
@@ -1711,7 +1713,7 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
     tm.collect();
     if (last_N < 0) return;
     IterResult& R = c->iters.back();
-    const double* avg = c->pin_avg.as<double>() + 8 * (last_N & 1);
+    const double* avg = c->pin_avg.as<double>() + kAvg * (last_N & 1);
     const double Zk = avg[last_avg];
     for (size_t k = 0; k < last_avg; ++k) R.opavg.push_back(std::fabs(Zk) < 1.e-20 ? avg[k] : avg[k] / Zk);
     float ms = 0.f;
@@ -1722,6 +1724,22 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
     t_last = now;
     last_N = -1;
   };
+  // A sweep that fails leaves the results of the iterations that did not: the last
+  // one's own error comes first, and without one it is finished.
+  auto settle_last = [&] {
+    if (last_N < 0 || cudaStreamSynchronize(c->stream) != cudaSuccess) return;
+    int f;
+    std::memcpy(&f, c->pin_avg.as<double>() + kAvg * (last_N & 1) + kAvg - 1, sizeof(int));
+    if (f == 0) {
+      finish_last();
+      return;
+    }
+    last_N = -1;
+    c->iters.pop_back();
+    if (dm) c->dm.pop_back();
+    check_flag_value(f);
+  };
+  try {  // up to the check after the loop
   for (int N = N0; N < cfg->nsites; ++N) {
     CU(cudaEventRecord(it0[N & 1], c->stream));
     IterResult R;
@@ -1863,8 +1881,9 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
     // The averages are read with the next iteration's results (finish_last), so
     // that the host builds that iteration's tables while this one's eigenvectors
     // and operators are computed.
-    double* const avg = c->pin_avg.as<double>() + 8 * (N & 1);
+    double* const avg = c->pin_avg.as<double>() + kAvg * (N & 1);
     CU(cudaMemcpyAsync(avg, c->scal.as<double>() + 24, sizeof(double) * 8, cudaMemcpyDeviceToHost, c->stream));
+    CU(cudaMemcpyAsync(avg + kAvg - 1, c->flag.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     c->timing.d2h_bytes += (int64_t)sizeof(double) * 8;
     tm.stop(to, &c->timing.cut_ms);
     // ---------------- tangents of this iteration (nrg_grad_forward)
@@ -2072,6 +2091,10 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
   CU(cudaEventRecord(span1, c->stream));
   CU(cudaEventSynchronize(span1));
   check_flag(c);
+  } catch (...) {
+    settle_last();
+    throw;
+  }
   finish_last();
   c->dm_spare.clear();
   float span_ms = 0.f;
