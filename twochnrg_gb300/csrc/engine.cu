@@ -62,6 +62,13 @@ struct DevBuf {
     CU(cudaMalloc(&p, want));
     cap = want;
   }
+  // Grows to just that: memory kept by the dozen.
+  void ensure_exact(size_t bytes) {
+    if (bytes <= cap) return;
+    if (p) { CU(cudaFree(p)); p = nullptr; cap = 0; }
+    CU(cudaMalloc(&p, bytes));
+    cap = bytes;
+  }
   void take(DevBuf& o) { std::swap(p, o.p); std::swap(cap, o.cap); }
   template <class T> T* as() const { return reinterpret_cast<T*>(p); }
 };
@@ -144,6 +151,11 @@ struct DmShell {
   std::vector<double> den;             // [p * nstates + i]: d en
   DevBuf dZ[4], dcd[4], drho[4];       // d Z (rows, the layout of Z), d c_d, d rho (the layout of rho)
   DevBuf ltpart;                       // tangent Lehmann partial sums, [p][the layout of lpart]
+  size_t device_bytes() const {
+    size_t n = Z.cap + cdel.cap + rho.cap + lpart.cap + ltpart.cap;
+    for (int p = 0; p < 4; ++p) n += dZ[p].cap + dcd[p].cap + drho[p].cap;
+    return n;
+  }
   // The device memory of a shell of the sweep before.
   void reuse(DmShell& o, bool tan) {
     Z.take(o.Z); cdel.take(o.cdel); rho.take(o.rho); lpart.take(o.lpart);
@@ -217,7 +229,10 @@ struct nrg_ctx {
   std::vector<std::unique_ptr<nrg::DmShell>> dm;
   // While a sweep that keeps shells runs: the shells of the one before, whose
   // device memory the new ones take over (40 shells' allocations and frees took
-  // 12 of a DM-NRG pass of 110 ms at 500 kept).  What is left is freed at its end.
+  // 12 of a DM-NRG pass of 110 ms at 500 kept), if it is at most kSpareBytes: larger
+  // ones are freed first, so that a sweep that fills the device still can.  What is
+  // left is freed at its end, or where it fails.
+  static constexpr size_t kSpareBytes = (size_t)2 << 30;
   std::vector<std::unique_ptr<nrg::DmShell>> dm_spare;
   bool dm_rho_valid = false;
   bool dm_drho_valid = false;          // the density matrices' tangents are built too
@@ -1563,13 +1578,16 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
     S.m.op_avg = {0, 0, 0};
   }
   if (dm) {
-    c->dm_spare = std::move(c->dm);
+    size_t held = 0;
+    for (const auto& s : c->dm) held += s->device_bytes();
+    if (held <= nrg_ctx::kSpareBytes) c->dm_spare = std::move(c->dm);
     c->dm.clear();
     c->dm_rho_valid = false;
     c->dm_drho_valid = false;
     c->dm_lambda = cfg->lambda;
     c->dm_model = S.m.kind;
   }
+  struct SpareGuard { nrg_ctx* c; ~SpareGuard() { c->dm_spare.clear(); } } spare{c};
   const ModelSpec& m = S.m;
   const double eps = cfg->degen_eps > 0 ? cfg->degen_eps : 1.0e-18;
   const double lambda = cfg->lambda;
@@ -2002,7 +2020,7 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
         shp->ntan = NP;
         shp->den.assign((size_t)(NP * ns), 0.0);
         for (int p = 0; p < NP; ++p) {
-          shp->dZ[p].ensure(sizeof(double) * ys);
+          shp->dZ[p].ensure_exact(sizeof(double) * ys);
           CU(cudaMemcpyAsync(shp->dZ[p].p, TS.dZ.as<double>() + p * ys, sizeof(double) * P.ysize,
                              cudaMemcpyDeviceToDevice, c->stream));
         }
@@ -2014,7 +2032,7 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
       if (dm) {
         const int64_t ncd = newops[nops_h].size;
         for (int p = 0; p < NP; ++p) {
-          shp->dcd[p].ensure(sizeof(double) * std::max<int64_t>(ncd, 1));
+          shp->dcd[p].ensure_exact(sizeof(double) * std::max<int64_t>(ncd, 1));
           CU(cudaMemcpyAsync(shp->dcd[p].p, op_tan(tnext, nops_h, p), sizeof(double) * ncd, cudaMemcpyDeviceToDevice,
                              c->stream));
         }
@@ -2062,9 +2080,9 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
       sh->kept_src = K.src;
       sh->cd = newops[nops_h];
       sh->zoff = P.yoff; sh->zsize = P.ysize;
-      sh->Z.ensure(sizeof(double) * std::max<int64_t>(P.ysize, 1));
+      sh->Z.ensure_exact(sizeof(double) * std::max<int64_t>(P.ysize, 1));
       CU(cudaMemcpyAsync(sh->Z.p, c->Z.p, sizeof(double) * P.ysize, cudaMemcpyDeviceToDevice, c->stream));
-      sh->cdel.ensure(sizeof(double) * std::max<int64_t>(newops[nops_h].size, 1));
+      sh->cdel.ensure_exact(sizeof(double) * std::max<int64_t>(newops[nops_h].size, 1));
       CU(cudaMemcpyAsync(sh->cdel.p, newptr[nops_h], sizeof(double) * newops[nops_h].size, cudaMemcpyDeviceToDevice,
                          c->stream));
       sh->basis = std::move(B);
@@ -2096,7 +2114,6 @@ void sweep_run(nrg_ctx* c, const nrg_sweep_config* cfg, bool dm = false, bool ch
     throw;
   }
   finish_last();
-  c->dm_spare.clear();
   float span_ms = 0.f;
   CU(cudaEventElapsedTime(&span_ms, span0, span1));
   c->timing.device_ms = span_ms;
@@ -2230,7 +2247,7 @@ void dm_backprop_impl(nrg_ctx* c, const nrg_dm_params* prm, double* rho_trace) {
       const int n = s.bsize[b];
       for (int i = 0; i < n; ++i) R[s.zoff[b] + (int64_t)i * n + i] = std::exp(-beta * s.en[s.boff[b] + i]) / ZTot;
     }
-    s.rho.ensure(sizeof(double) * R.size());
+    s.rho.ensure_exact(sizeof(double) * R.size());
     h2d(c, s.rho.p, R.data(), sizeof(double) * s.zsize);
     s.rrows.assign(s.bsize.size(), 0);
     for (size_t b = 0; b < s.bsize.size(); ++b) {
@@ -2248,7 +2265,7 @@ void dm_backprop_impl(nrg_ctx* c, const nrg_dm_params* prm, double* rho_trace) {
           dR[q] = R[q] * (-beta * dE[s.boff[b] + i] - dlogz[k]);
         }
       }
-      s.drho[k].ensure(sizeof(double) * dR.size());
+      s.drho[k].ensure_exact(sizeof(double) * dR.size());
       h2d(c, s.drho[k].p, dR.data(), sizeof(double) * s.zsize);
     }
   }
@@ -2333,7 +2350,7 @@ void dm_backprop_impl(nrg_ctx* c, const nrg_dm_params* prm, double* rho_trace) {
     c->meta.ensure(pk.host.size() + 256);
     h2d(c, c->meta.p, pk.host.data(), pk.host.size());
     char* mb = c->meta.as<char>();
-    sN.rho.ensure(sizeof(double) * std::max<int64_t>(sN.zsize, 1));
+    sN.rho.ensure_exact(sizeof(double) * std::max<int64_t>(sN.zsize, 1));
     TempBar = p.temp / calc_dn(L, N - 1);
     DmTraceArgs ta{};
     ta.bsize = (const int*)(mb + o_bs); ta.soff = (const int*)(mb + o_so); ta.roff = (const int64_t*)(mb + o_ro);
@@ -2359,7 +2376,7 @@ void dm_backprop_impl(nrg_ctx* c, const nrg_dm_params* prm, double* rho_trace) {
       tt.rot = (const double*)((char*)U0 + (DmTan::NP + k) * zsa);
       tt.dE = (const double*)(mb + o_den) + (size_t)k * sN.en.size();
       tt.dlogz = dlogz[k];
-      sN.drho[k].ensure(sizeof(double) * std::max<int64_t>(sN.zsize, 1));
+      sN.drho[k].ensure_exact(sizeof(double) * std::max<int64_t>(sN.zsize, 1));
       tt.rho = sN.drho[k].as<double>();
       launch_dm_trace(tt, nbN, c->stream);
       c->launches++;
@@ -2692,8 +2709,8 @@ void lehmann_impl(nrg_ctx* c, const nrg_dm_params* prm, int nomega, const double
       sl_off.push_back(part - nchk * li.nomega);
     }
     if (items.size() > (size_t)INT32_MAX) throw NrgError(NRG_ERR_SIZE, "too many Lehmann work items");
-    s.lpart.ensure(sizeof(double) * std::max<int64_t>(part, 1));
-    if (tg) s.ltpart.ensure(sizeof(double) * std::max<int64_t>(NP * part, 1));
+    s.lpart.ensure_exact(sizeof(double) * std::max<int64_t>(part, 1));
+    if (tg) s.ltpart.ensure_exact(sizeof(double) * std::max<int64_t>(NP * part, 1));
     std::vector<LehList> stl;  // this shell's tangent lists, parameter major
     for (int k = 0; tg && k < NP; ++k)
       for (size_t q = 0; q < sl.size(); ++q) {
