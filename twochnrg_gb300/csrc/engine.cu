@@ -451,9 +451,11 @@ int rows_block_threshold() {
 // 1.34, 2.15 ms), 8 for smaller blocks, where the CTAs would have one row or
 // none (32 states: 64 us on 8, 67 on 16).  Also for the workers of
 // nrg_sweep_batch (16 sweeps: 1.27 s on 16, 1.35 on 8, 1.33 on 4, 1.40 on 2).
+// NRG_ROWS_CLUSTER sets it; what is no cluster size is ignored.
 int choose_rows_cluster(int maxn) {
   const char* s = std::getenv("NRG_ROWS_CLUSTER");
-  if (s) return std::atoi(s);
+  const int c = s ? std::atoi(s) : 0;
+  if (c == 1 || c == 2 || c == 4 || c == 8 || c == 16) return c;
   return maxn > 32 ? 16 : 8;
 }
 
@@ -860,7 +862,8 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
     const int maxs = std::max(P.bsize[order_h[nrows0]], 2);
     rcl = choose_rows_cluster(maxs);
     rncl = tridiag_rows_max_clusters(rcl, maxs);
-    for (; rncl <= 0 && rcl < 16; ) { rcl *= 2; rncl = tridiag_rows_max_clusters(rcl, maxs); }
+    while (rncl <= 0 && rcl < 16) { rcl *= 2; rncl = tridiag_rows_max_clusters(rcl, maxs); }
+    if (rncl <= 0) { rcl = 8; rncl = tridiag_rows_max_clusters(rcl, maxs); }  // no clusters of 16 to be had
     if (rncl > 0) break;
   }
   const int nmid = nrows0 - nbig - nspan;
