@@ -138,8 +138,7 @@ __device__ inline RowsSm rows_carve(double* sm, int maxn, int cl) {
 // RT of the CTA's rows: the pending update A - p y^T - q u^T and the product with
 // x over columns j+1..n-1.
 template <int RT>
-__device__ __forceinline__ void sweep_rows(const RowsSm& S, int CL, int rank, int n, int j, int i0, const double* xc,
-                                           const double* uo) {
+__device__ __forceinline__ void sweep_rows(const RowsSm& S, int n, int j, int i0, const double* xc, const double* uo) {
   const int lane = threadIdx.x & 31;
   double* row = S.rows + i0 * S.ld;
   const int step = kSweep * S.ld;
@@ -306,9 +305,9 @@ __global__ void __launch_bounds__(kRowsThreads, 3) tridiag_rows_kernel(TridiagAr
       } else {
         int i = i0 + warp;
 #pragma unroll 1
-        for (; i + 3 * kSweep < own; i += 4 * kSweep) sweep_rows<4>(S, CL, rank, n, j, i, xc, uo);
-        if (i + kSweep < own) { sweep_rows<2>(S, CL, rank, n, j, i, xc, uo); i += 2 * kSweep; }
-        if (i < own) sweep_rows<1>(S, CL, rank, n, j, i, xc, uo);
+        for (; i + 3 * kSweep < own; i += 4 * kSweep) sweep_rows<4>(S, n, j, i, xc, uo);
+        if (i + kSweep < own) { sweep_rows<2>(S, n, j, i, xc, uo); i += 2 * kSweep; }
+        if (i < own) sweep_rows<1>(S, n, j, i, xc, uo);
       }
       __syncthreads();
       // (y, next column) of the own rows to every CTA; tau meanwhile.

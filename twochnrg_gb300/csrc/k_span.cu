@@ -107,9 +107,8 @@ enum { SC_BETA, SC_TU1, SC_B, SC_H2 };
 // and the product with x over strips s0 .. s1-1 of columns j+1..n-1, whose sums
 // go to out[k * od].
 template <int RT>
-__device__ __forceinline__ void span_rows(const SpanSm& S, double* row, int64_t ld, int G, int rank, int n, int j, int i0,
-                                          int di, int s0, int s1, double* out, int od, const double* xc,
-                                          const double* uo) {
+__device__ __forceinline__ void span_rows(const SpanSm& S, double* row, int64_t ld, int n, int j, int i0, int di, int s0,
+                                          int s1, double* out, int od, const double* xc, const double* uo) {
   const int lane = threadIdx.x & 31, step = (int)(di * ld);
   double p[RT], q[RT], acc[RT];
 #pragma unroll
@@ -159,31 +158,31 @@ __device__ __forceinline__ void span_rows(const SpanSm& S, double* row, int64_t 
 }
 
 // The warp's rows among own rows [first, end): `base` is own row i = 0's place.
-__device__ __forceinline__ void span_sweep(const SpanSm& S, double* base, int64_t ld, int first, int end, int G, int rank,
-                                           int n, int j, const double* xc, const double* uo) {
+__device__ __forceinline__ void span_sweep(const SpanSm& S, double* base, int64_t ld, int first, int end, int n, int j,
+                                           const double* xc, const double* uo) {
   const int warp = threadIdx.x >> 5, ns = (n - j - 1 + 31) >> 5;
   int i = first + warp;
 #pragma unroll 1
   for (; i + 3 * kSweep < end; i += 4 * kSweep)
-    span_rows<4>(S, base + i * ld, ld, G, rank, n, j, i, kSweep, 0, ns, S.tot + i, kSweep, xc, uo);
+    span_rows<4>(S, base + i * ld, ld, n, j, i, kSweep, 0, ns, S.tot + i, kSweep, xc, uo);
   if (i + kSweep < end) {
-    span_rows<2>(S, base + i * ld, ld, G, rank, n, j, i, kSweep, 0, ns, S.tot + i, kSweep, xc, uo);
+    span_rows<2>(S, base + i * ld, ld, n, j, i, kSweep, 0, ns, S.tot + i, kSweep, xc, uo);
     i += 2 * kSweep;
   }
-  if (i < end) span_rows<1>(S, base + i * ld, ld, G, rank, n, j, i, kSweep, 0, ns, S.tot + i, kSweep, xc, uo);
+  if (i < end) span_rows<1>(S, base + i * ld, ld, n, j, i, kSweep, 0, ns, S.tot + i, kSweep, xc, uo);
 }
 // Own rows [first, end), at most kSweep - 1: every warp takes a quarter of the
 // columns.
-__device__ __forceinline__ void span_split(const SpanSm& S, double* base, int64_t ld, int first, int end, int G, int rank,
-                                           int n, int j, const double* xc, const double* uo) {
+__device__ __forceinline__ void span_split(const SpanSm& S, double* base, int64_t ld, int first, int end, int n, int j,
+                                           const double* xc, const double* uo) {
   const int warp = threadIdx.x >> 5, ns = (n - j - 1 + 31) >> 5;
   const int s0 = ns * warp / kSweep, s1 = ns * (warp + 1) / kSweep;
   int i = first;
   if (i + 1 < end) {
-    span_rows<2>(S, base + i * ld, ld, G, rank, n, j, i, 1, s0, s1, S.quart + warp, kSweep, xc, uo);
+    span_rows<2>(S, base + i * ld, ld, n, j, i, 1, s0, s1, S.quart + warp, kSweep, xc, uo);
     i += 2;
   }
-  if (i < end) span_rows<1>(S, base + i * ld, ld, G, rank, n, j, i, 1, s0, s1, S.quart + (i - first) * kSweep + warp, kSweep, xc, uo);
+  if (i < end) span_rows<1>(S, base + i * ld, ld, n, j, i, 1, s0, s1, S.quart + (i - first) * kSweep + warp, kSweep, xc, uo);
 }
 
 // The gathered y and the first part of the next x, L entries per thread in flight
@@ -285,7 +284,7 @@ __global__ void __launch_bounds__(kSpanThreads, 1) tridiag_span_kernel(TridiagAr
     double* gbase = H + (int64_t)rank * n;
     const int64_t gld = (int64_t)G * n;
     double* sbase = S.rows - (int64_t)ng * S.ld;
-    for (int i = ng + warp; i < own; i += kSweep + 1) {
+    for (int i = ng + warp; i < own; i += kSpanThreads / 32) {
       const double* src = gbase + i * gld;
       double* dst = sbase + i * S.ld;
       for (int c = lane; c < n; c += 32) dst[c] = __ldcg(src + c);
@@ -361,9 +360,9 @@ __global__ void __launch_bounds__(kSpanThreads, 1) tridiag_span_kernel(TridiagAr
         if (lane < R) store_share(E.share + (size_t)((g + 1) % kBufs + kBufs * lane) * G + rank, empty);
         asm volatile("fence.acq_rel.gpu;" ::: "memory");
       } else {
-        if (i0 < ng) span_sweep(S, gbase, gld, i0, ng, G, rank, n, j, xc, uo);
-        span_sweep(S, sbase, S.ld, max(i0, ng), isplit, G, rank, n, j, xc, uo);
-        if (isplit < own) span_split(S, sbase, S.ld, isplit, own, G, rank, n, j, xc, uo);
+        if (i0 < ng) span_sweep(S, gbase, gld, i0, ng, n, j, xc, uo);
+        span_sweep(S, sbase, S.ld, max(i0, ng), isplit, n, j, xc, uo);
+        if (isplit < own) span_split(S, sbase, S.ld, isplit, own, n, j, xc, uo);
       }
       __syncthreads();
       if (warp == kSweep) {
