@@ -17,8 +17,8 @@ namespace nrg {
 
 namespace {
 
-// TAN: direction blockIdx.y of the tangent pass, with Zt's tangent into T's (the
-// site-operator terms; the old operators' terms are imp_gemm_kernel's).
+// The site-operator terms (the old operators' are imp_gemm_kernel's).  TAN:
+// direction blockIdx.y of the tangent pass, with Zt's tangent into T's.
 template <bool TAN>
 __global__ void __launch_bounds__(256) gather_kernel(UpdateArgs A) {
   const int g = blockIdx.x;
@@ -31,23 +31,10 @@ __global__ void __launch_bounds__(256) gather_kernel(UpdateArgs A) {
     const int kj = J.kj;
     double* T = Tall + J.t_off;
     const double* Zt = Zall + J.zt_off;
-    if (G.mode == 0) {
-      for (int idx = threadIdx.x; idx < G.rows * kj; idx += blockDim.x) {
-        const int a = idx / kj, c = idx - a * kj;
-        double* dst = T + (int64_t)(G.dst_base + a * G.dst_stride) * kj + c;
-        *dst = fma(G.coef, Zt[(int64_t)(G.src_base + a * G.src_stride) * J.ldz + c], *dst);
-      }
-    } else {
-      const double* M = A.old_ops[G.op] + G.old_off;
-      for (int idx = threadIdx.x; idx < G.rows * kj; idx += blockDim.x) {
-        const int a = idx / kj, c = idx - a * kj;
-        double acc = 0.0;
-        const double* Ma = M + (int64_t)a * G.old_ld;
-        for (int bb = 0; bb < G.srows; ++bb)
-          acc = fma(Ma[bb], Zt[(int64_t)(G.src_base + bb * G.src_stride) * J.ldz + c], acc);
-        double* dst = T + (int64_t)(G.dst_base + a * G.dst_stride) * kj + c;
-        *dst = fma(G.coef, acc, *dst);
-      }
+    for (int idx = threadIdx.x; idx < G.rows * kj; idx += blockDim.x) {
+      const int a = idx / kj, c = idx - a * kj;
+      double* dst = T + (int64_t)(G.dst_base + a * G.dst_stride) * kj + c;
+      *dst = fma(G.coef, Zt[(int64_t)(G.src_base + a * G.src_stride) * J.ldz + c], *dst);
     }
     __syncthreads();
   }

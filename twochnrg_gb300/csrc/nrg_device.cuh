@@ -217,7 +217,6 @@ struct TridiagArgs {
 cudaError_t launch_tridiag(const TridiagArgs& a, int cluster, int nclusters, cudaStream_t s, int threads = 512);
 size_t tridiag_smem_bytes(int maxn, int cluster, int threads = 512);
 int tridiag_max_clusters(int cluster, int maxn, int threads = 512);
-// Blocks whose rows fit in a cluster's shared memory (k_rows.cu).
 // One block per group of G CTAs, the groups' blocks in list[first[g]] ..
 // list[first[g + 1]) (k_span.cu).  A cooperative launch; work:
 // tridiag_span_work(maxn, groups, G, copies) doubles.
@@ -232,6 +231,7 @@ struct SpanArgs {
 size_t tridiag_span_work(int maxn, int groups, int G, int copies);
 bool tridiag_span_fits(int n);        // its vectors fit in shared memory
 cudaError_t launch_tridiag_span(const TridiagArgs& a, SpanArgs p, int groups, cudaStream_t s);
+// Blocks whose rows fit in a cluster's shared memory (k_rows.cu).
 size_t tridiag_rows_smem_bytes(int maxn, int cluster);
 int tridiag_rows_max_clusters(int cluster, int maxn);
 cudaError_t launch_tridiag_rows(const TridiagArgs& a, int cluster, int nclusters, cudaStream_t s);
@@ -354,7 +354,7 @@ struct GatherTerm {       // T[dst rows] += coef * M . Zt[src rows]
   int job;                // rotation job
   int dst_base, dst_stride, rows;   // rows of T (local to the job's T)
   int src_base, src_stride, srows;  // rows of Zt_J (local to block J)
-  int mode;               // 0: identity (srows == rows); 1: old block (rows x srows)
+  int mode;               // 0: identity (srows == rows), in terms; 1: old block (rows x srows), in terms1
   double coef;
   int64_t old_off;        // element offset of the old block (mode 1)
   int old_ld;             // its row stride (columns of the stored old block)
