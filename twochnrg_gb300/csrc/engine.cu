@@ -348,11 +348,12 @@ void stream_wait(nrg_ctx* c) {
 }
 
 void check_flag_value(int f) {
+  // first: every value after a wait that gave up is void
+  if (f & DEV_TIMEOUT) throw NrgError(NRG_ERR_TIMEOUT, "a kernel's bounded wait gave up");
   if (f & DEV_SIZE) throw NrgError(NRG_ERR_SIZE, "a block exceeds the eigensolver size limit");
   if (f & DEV_DEGEN_OVERFLOW) throw NrgError(NRG_ERR_SIZE, "too many near-degenerate levels for SetDegen");
   if (f & DEV_BAD_INPUT) throw NrgError(NRG_ERR_ARG, "non-finite value met in an eigenvalue solve");
   if (f & DEV_NOT_CONVERGED) throw NrgError(NRG_ERR_NOT_CONVERGED, "inverse iteration did not converge");
-  if (f & DEV_TIMEOUT) throw NrgError(NRG_ERR_TIMEOUT, "a kernel's bounded wait gave up");
 }
 void check_flag(nrg_ctx* c) {
   int f = 0;
@@ -618,6 +619,11 @@ std::vector<std::vector<int>> deal_by_cost(const std::vector<int>& blocks, const
 int span_from() {
   const char* s = std::getenv("NRG_SPAN_N");
   return s ? std::atoi(s) : 450;
+}
+// About two seconds; a test makes a wait run out with less.
+long long span_wait_cycles() {
+  const char* s = std::getenv("NRG_SPAN_WAIT");
+  return s ? std::atoll(s) : 4000000000ll;
 }
 constexpr int kSpanCopies = 4;     // of its exchange area (1901 states on 152 CTAs: 28.4 ms with 1, 26.7 with 4)
 constexpr int kGridFrom = 1200;    // smallest block considered for the whole-GPU kernel beside span groups
@@ -911,6 +917,7 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
     SpanArgs sa{};
     sa.list = (const int*)(c->slist.as<char>() + o_span); sa.first = (const int*)(c->slist.as<char>() + o_sfirst);
     sa.work = c->swork.as<double>(); sa.G = sp.G; sa.copies = kSpanCopies;
+    sa.wait_cycles = span_wait_cycles();
     TridiagArgs ts = ta;
     ts.maxn = P.bsize[order_h[nbig]];
     CU(launch_tridiag_span(ts, sa, sp.groups, ss));

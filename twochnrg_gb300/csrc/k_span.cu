@@ -49,7 +49,6 @@ constexpr int kSplitCols = 128;                  // at least a strip of columns 
 constexpr int kPollCols = 768;                   // from here on the gather waits for the shares
 constexpr int kBufs = 3;
 constexpr long long kEmpty = -1;                 // a NaN that no FP64 operation gives
-constexpr long long kWaitCycles = 4000000000ll;  // about two seconds
 
 __device__ __forceinline__ double2 load_pair(const double2* p) {
   double2 v;
@@ -189,7 +188,7 @@ __device__ __forceinline__ void span_split(const SpanSm& S, double* base, int64_
 // (a round trip through L2 each).
 template <int L>
 __device__ __forceinline__ void gather(const SpanSm& S, const double2* pair, int j, int n, double tu1, double* uo,
-                                       volatile int* dead, int* flag) {
+                                       volatile int* dead, int* flag, long long limit) {
 #pragma unroll 1
   for (int c = j + 1 + (int)threadIdx.x; c < n; c += L * kSweep * 32) {
     double2 v[L];
@@ -202,7 +201,7 @@ __device__ __forceinline__ void gather(const SpanSm& S, const double2* pair, int
       if (!is_full(v[k]) && !*dead) {
         const long long t0 = clock64();
         do {
-          if (clock64() - t0 > kWaitCycles) { *dead = 1; atomicOr(flag, DEV_TIMEOUT); }
+          if (clock64() - t0 > limit) { *dead = 1; atomicOr(flag, DEV_TIMEOUT); }
           v[k] = load_pair(pair + ck);
         } while (!is_full(v[k]) && !*dead);
       }
@@ -213,7 +212,8 @@ __device__ __forceinline__ void gather(const SpanSm& S, const double2* pair, int
 }
 
 // Barrier of the group: every CTA arrives once per call.
-__device__ __forceinline__ void group_barrier(const SpanEx& E, unsigned target, volatile int* dead, int* flag) {
+__device__ __forceinline__ void group_barrier(const SpanEx& E, unsigned target, volatile int* dead, int* flag,
+                                              long long limit) {
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
@@ -223,7 +223,7 @@ __device__ __forceinline__ void group_barrier(const SpanEx& E, unsigned target, 
       unsigned v;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(E.count) : "memory");
       if (v >= target) break;
-      if (clock64() - t0 > kWaitCycles) { *dead = 1; atomicOr(flag, DEV_TIMEOUT); }
+      if (clock64() - t0 > limit) { *dead = 1; atomicOr(flag, DEV_TIMEOUT); }
     }
     __threadfence();
   }
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(kSpanThreads, 1) tridiag_span_kernel(TridiagAr
       S.y[c] = 0.0;
     }
     for (int i = tid; i < own; i += kSpanThreads) S.p[i] = S.q[i] = 0.0;
-    group_barrier(E, arrived += G, dead, A.flag);  // row 0 is read before it is overwritten
+    group_barrier(E, arrived += G, dead, A.flag, P.wait_cycles);  // row 0 is read before it is overwritten
     if (warp < kSweep) {  // norm partials of the first x (elements 2..n-1)
       double s = 0.0;
       for (int c = 2 + tid; c < n; c += kSweep * 32) s = fma(S.x[c], S.x[c], s);
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(kSpanThreads, 1) tridiag_span_kernel(TridiagAr
           double va = load_share(share + qa), vb = load_share(share + qb);
           const long long t0 = clock64();
           while (!(is_full(va) && is_full(vb)) && !*dead) {
-            if (clock64() - t0 > kWaitCycles) { *dead = 1; atomicOr(A.flag, DEV_TIMEOUT); }
+            if (clock64() - t0 > P.wait_cycles) { *dead = 1; atomicOr(A.flag, DEV_TIMEOUT); }
             va = load_share(share + qa);
             vb = load_share(share + qb);
           }
@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(kSpanThreads, 1) tridiag_span_kernel(TridiagAr
         if (!is_full(v1) && !*dead) {
           const long long t0 = clock64();
           do {
-            if (clock64() - t0 > kWaitCycles) { *dead = 1; atomicOr(A.flag, DEV_TIMEOUT); }
+            if (clock64() - t0 > P.wait_cycles) { *dead = 1; atomicOr(A.flag, DEV_TIMEOUT); }
             v1 = load_pair(pair + j + 1);
           } while (!is_full(v1) && !*dead);
         }
@@ -430,9 +430,9 @@ __global__ void __launch_bounds__(kSpanThreads, 1) tridiag_span_kernel(TridiagAr
         // / 3.03, 3.14, 3.20 ms; after the shares 8 deep 25.0 / 6.85 / 3.11 ms.
         if (m > kPollCols) {
           asm volatile("barrier.cta.sync 1, %0;" ::"n"((kSweep + 1) * 32) : "memory");
-          gather<8>(S, pair, j, n, tu1, uo, dead, A.flag);
+          gather<8>(S, pair, j, n, tu1, uo, dead, A.flag, P.wait_cycles);
         } else {
-          gather<2>(S, pair, j, n, tu1, uo, dead, A.flag);
+          gather<2>(S, pair, j, n, tu1, uo, dead, A.flag, P.wait_cycles);
         }
       }
       __syncthreads();
@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(kSpanThreads, 1) tridiag_span_kernel(TridiagAr
       A.tau[so + n - 1] = 0.0;
     }
     // All gathers are done: empty the own entries for the next block.
-    group_barrier(E, arrived += G, dead, A.flag);
+    group_barrier(E, arrived += G, dead, A.flag, P.wait_cycles);
     const double empty = __longlong_as_double(kEmpty);
     for (int k = tid; k < kBufs * R * own; k += kSpanThreads)
       store_pair(E.pair + (size_t)(k / own) * A.maxn + rank + G * (k % own), empty, empty);

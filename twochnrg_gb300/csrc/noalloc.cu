@@ -177,9 +177,9 @@ extern "C" nrg_status nrg_diag_block_noalloc(int n, const double* a, double* eig
   int flag = 0;
   if (cudaMemcpyAsync(&flag, L.flag, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess) return NRG_ERR_CUDA;
   if (cudaStreamSynchronize(s) != cudaSuccess) return NRG_ERR_CUDA;
+  if (flag & DEV_TIMEOUT) return NRG_ERR_TIMEOUT;  // first: every value after it is void
   if (flag & DEV_SIZE) return NRG_ERR_SIZE;
   if (flag & DEV_BAD_INPUT) return NRG_ERR_ARG;
   if (flag & DEV_NOT_CONVERGED) return NRG_ERR_NOT_CONVERGED;
-  if (flag & DEV_TIMEOUT) return NRG_ERR_TIMEOUT;
   return NRG_OK;
 }

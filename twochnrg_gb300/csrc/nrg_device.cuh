@@ -226,6 +226,7 @@ struct SpanArgs {
   double* work;
   int G;
   int copies;        // of the exchange area, each read by every copies-th CTA (up to 32)
+  long long wait_cycles;  // a wait gives up after so many SM clocks
   int smem_doubles;  // set by the launch
 };
 size_t tridiag_span_work(int maxn, int groups, int G, int copies);
