@@ -510,7 +510,20 @@ void ensure_second_stream(nrg_ctx* c) {
 // other.  A context holds this lock from the launch of its grids until they
 // have finished; the launches of other contexts' non-cooperative kernels are
 // not held up.
+// A way out by an exception waits for what was launched too.
 std::mutex g_coop_mu;
+struct CoopLock {
+  nrg_ctx* c;
+  std::unique_lock<std::mutex> lock{g_coop_mu, std::defer_lock};
+  explicit CoopLock(nrg_ctx* ctx) : c(ctx) {}
+  ~CoopLock() {
+    if (!lock.owns_lock()) return;
+    cudaStreamSynchronize(c->stream);
+    if (c->rows_stream) cudaStreamSynchronize(c->rows_stream);
+    for (cudaStream_t s : c->aux)
+      if (s) cudaStreamSynchronize(s);
+  }
+};
 
 // Panel width of the blocked reduction (mixed precision): the trailing
 // product has K = 2 nb.
@@ -777,9 +790,9 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
     c->swork.ensure(sizeof(double) * tridiag_span_work(P.bsize[order_h[nbig]], sp.groups, sp.G, kSpanCopies));
     if (!c->span_join) CU(cudaEventCreateWithFlags(&c->span_join, cudaEventDisableTiming));
   }
-  std::unique_lock<std::mutex> coop(g_coop_mu, std::defer_lock);
+  CoopLock coop(c);
   if (K >= 1 || nspan > 0) {
-    coop.lock();
+    coop.lock.lock();
     for (int k = 0; k < K; ++k)
       if (!c->join[k]) CU(cudaEventCreateWithFlags(&c->join[k], cudaEventDisableTiming));
   }
@@ -948,10 +961,10 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
     }
   }
   for (int k = 0; K > 1 && k < K; ++k) CU(cudaStreamWaitEvent(c->stream, c->join[k], 0));
-  if (coop.owns_lock()) {
+  if (coop.lock.owns_lock()) {
     for (int k = 0; k < K; ++k) CU(cudaEventSynchronize(c->join[k]));
     if (nspan > 0) CU(cudaEventSynchronize(c->span_join));
-    coop.unlock();
+    coop.lock.unlock();
   }
   tm.stop(t0, &c->timing.tridiag_ms);
   double fl = 0.0;
