@@ -9,8 +9,8 @@
 //   exp(-(tau - s)^2) = sum_n (s/r)^n b_n(tau),  b_n = r^n H_n(tau) exp(-tau^2) / n!
 // (the generating function of the Hermite polynomials H_n), so that a bin
 // is its kTerms moments sum_i w_i (s_i/r)^n and a record costs two operations
-// per moment, once: 10.7 ms for the same sums, 6.7 of it the moments, 2.0 their
-// evaluation.  Lists of the tangents use
+// per moment, once: 10.7 ms for the same sums, most of it the moments (about 6.5)
+// and their evaluation (2.0).  Lists of the tangents use
 // (tau - s) exp(-(tau - s)^2) = sum_n (s/r)^n (n+1)/(2r) b_{n+1}(tau).
 //
 // What is dropped, and what is rounded.  With r = 1/16 and 28 terms the first
@@ -165,18 +165,15 @@ __global__ void __launch_bounds__(kWarps * 32) fgt_moments_kernel(const FgtList*
       v *= u;
     }
   }
-  const int warps = min(kWarps, (s1 - s0 + 31) >> 5);  // with records
-  if (warp < warps) {
 #pragma unroll
-    for (int n = 0; n < kTerms; ++n) {
-      const double v = warp_sum_fixed(m[n]);
-      if (lane == 0) part[warp][n] = v;
-    }
+  for (int n = 0; n < kTerms; ++n) {
+    const double v = warp_sum_fixed(m[n]);
+    if (lane == 0) part[warp][n] = v;
   }
   __syncthreads();
   if (threadIdx.x < kTerms) {
     double v = 0.0;
-    for (int q = 0; q < warps; ++q) v += part[q][threadIdx.x];
+    for (int q = 0; q < kWarps; ++q) v += part[q][threadIdx.x];
     if (set > 0 && !(set & 1)) v *= (threadIdx.x + 1) * (1.0 / (2.0 * kR));
     L.moments[((int64_t)set * kTerms + threadIdx.x) * L.nbins + b] = v;
   }
