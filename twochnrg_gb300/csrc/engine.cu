@@ -6,9 +6,9 @@
 // The host does the block bookkeeping (a few hundred blocks) and builds the
 // small tables the kernels read; everything per state and per matrix element
 // runs on the device, and the kept eigenvectors and operator blocks stay in
-// HBM from one iteration to the next.  Two host synchronisations per
-// iteration remain: after the cut (the kept counts shape the next launches)
-// and after the operator averages.
+// HBM from one iteration to the next.  The host waits once per iteration, after
+// the cut (the kept counts shape the next launches), and reads the operator
+// averages with the next iteration's results.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -2455,9 +2455,9 @@ std::vector<double> dm_grid(double L, int nsh, int nw) {
 // Lists from this many records on are summed through the moments of key bins
 // (k_fgt.cu); shorter ones, or ones whose keys span more bins than it has,
 // directly.  One-channel spectral function at 500 kept and 2000 frequencies:
-// the sums take 9.3 / 9.9 / 9.5 ms from 256 / 1024 / 4096 records on and 195 ms
-// directly; with four tangents at 200 kept and 512 frequencies the whole
-// spectral part 17.5 / 18.1 / 22.9 ms and 103 ms.
+// the sums take 10.7 / 10.9 ms from 256 / 1024 records on and 195 ms directly; with
+// four tangents at 200 kept and 512 frequencies the whole spectral part 11.0 / 11.6
+// ms (16.3 from 4096 on) and 103 ms.
 int64_t fgt_min_records() {
   const char* s = std::getenv("NRG_FGT_MIN");
   return s ? std::atoll(s) : 256;
