@@ -7,7 +7,7 @@ The number of lanes follows from the rows of all blocks against the device's
 lanes; the copies of each list are chosen so that every kernel takes its turn,
 and the rule is asserted.  Bounds, in ulps of the spectral radius' bound: a level
 stands alone within 8 (the bracket's end) and the counts' own error, 16; of a
-pair or triple, 8 and 4 lanes certify it 7 from their last point on either side:
+pair or triple, 8 and 4 lanes end at a bracket of 19 and the counts' own error:
 24; one lane accepts a resolved pair's step (16 and 8 from the counts) and a
 group within 64: 24 and 72."""
 import numpy as np
