@@ -536,17 +536,25 @@ constexpr int kOzSlices = 6;
 // trailing rank-2 kPanelNb update H[k1:, k1:] -= [V W] [W V]^T as an
 // FP64-accurate split-BF16 product on the tensor cores (k_ozaki.cu), limited
 // to G CTAs so that concurrent grids share the GPU evenly.
-void blocked_reduction(nrg_ctx* c, const EigPlan& P, const std::vector<int>& blocks, int slot, int G,
-                       cudaStream_t s) {
-  const int nb = kPanelNb, ld = 2 * kPanelNb;
+// blocked_scratch comes first, for every stream before the first launch.
+int blocked_maxn(const EigPlan& P, const std::vector<int>& blocks) {
   int maxn = 3;
   for (int b : blocks) maxn = std::max(maxn, P.bsize[b]);
+  return maxn;
+}
+void blocked_scratch(nrg_ctx* c, const EigPlan& P, const std::vector<int>& blocks, int slot, int G) {
+  const int ld = 2 * kPanelNb;
   // sized for the next multiple of 1024 states: the largest block creeps up
   // over a sweep, and a reallocation synchronises the device
-  const size_t nres = ((size_t)maxn + 1023) / 1024 * 1024;
+  const size_t nres = ((size_t)blocked_maxn(P, blocks) + 1023) / 1024 * 1024;
   c->pvw[slot].ensure(sizeof(double) * nres * ld);
   c->pcol[slot].ensure(sizeof(double) * (2 * nres + 2 + (size_t)G * (ld + 2)));
   c->ozk[slot].ensure(oz_work_bytes((int)nres, (int)nres, ld, kOzSlices));
+}
+void blocked_reduction(nrg_ctx* c, const EigPlan& P, const std::vector<int>& blocks, int slot, int G,
+                       cudaStream_t s) {
+  const int nb = kPanelNb, ld = 2 * kPanelNb;
+  const int maxn = blocked_maxn(P, blocks);
   double* VW = c->pvw[slot].as<double>();
   double* col = c->pcol[slot].as<double>();
   double* ybuf = col + 2 * (size_t)maxn;
@@ -790,6 +798,11 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
     c->swork.ensure(sizeof(double) * tridiag_span_work(P.bsize[order_h[nbig]], sp.groups, sp.G, kSpanCopies));
     if (!c->span_join) CU(cudaEventCreateWithFlags(&c->span_join, cudaEventDisableTiming));
   }
+  // What the kernels below read and write is there before the first of them runs: a
+  // buffer that grows is freed first, and that waits for the whole device, so that
+  // one of four concurrent grids waited for the one before it (a sweep's first
+  // iteration at 1500 kept 600 ms in place of 200).
+  c->rlist.ensure(sizeof(int) * (2 * (size_t)nb + 2) + 1024);
   CoopLock coop(c);
   if (K >= 1 || nspan > 0) {
     coop.lock.lock();
@@ -830,6 +843,10 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
       for (int b : bins[k]) (P.bsize[b] >= mthr ? bl[k] : fp[k]).push_back(b);
       o_fp[k] = pk.add(fp[k]);
     }
+    for (int k = 0; k < K; ++k) {
+      if (!fp[k].empty()) c->gpart_k[k].ensure(sizeof(double) * tridiag_grid_work(ta.maxn, Gfp / K));
+      if (!bl[k].empty()) blocked_scratch(c, P, bl[k], k, G / K);
+    }
     c->gbig.ensure(pk.host.size() + 256);
     h2d(c, c->gbig.p, pk.host.data(), pk.host.size());
     if (!c->fork) CU(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
@@ -842,7 +859,6 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
         CU(cudaStreamWaitEvent(sk, c->fork, 0));
       }
       if (!fp[k].empty()) {
-        c->gpart_k[k].ensure(sizeof(double) * tridiag_grid_work(ta.maxn, Gfp / K));
         CU(launch_tridiag_grid(ta, (const int*)(c->gbig.as<char>() + o_fp[k]), (int)fp[k].size(),
                                c->gpart_k[k].as<double>(), Gfp / K, sk));
         c->launches++; c->timing.tridiag_launches++;
@@ -861,11 +877,11 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
     const int G = tridiag_grid_size(ta.maxn);
     if (G <= 0) throw NrgError(NRG_ERR_SIZE, "whole-GPU tridiagonalization does not fit");
     const int Gk = G / K;
+    for (int k = 0; k < K; ++k) c->gpart_k[k].ensure(sizeof(double) * tridiag_grid_work(ta.maxn, Gk));
     if (!c->fork) CU(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
     CU(cudaEventRecord(c->fork, c->stream));
     for (int k = 0; k < K; ++k) {
       if (!c->aux[k]) CU(cudaStreamCreateWithFlags(&c->aux[k], cudaStreamNonBlocking));
-      c->gpart_k[k].ensure(sizeof(double) * tridiag_grid_work(ta.maxn, Gk));
       CU(cudaStreamWaitEvent(c->aux[k], c->fork, 0));
       CU(launch_tridiag_grid(ta, (const int*)(c->gbig.as<char>() + o_bins[k]), (int)bins[k].size(),
                              c->gpart_k[k].as<double>(), Gk, c->aux[k]));
@@ -890,6 +906,8 @@ void run_tridiag_and_bisect(nrg_ctx* c, Timer& tm, const EigPlan& P, const std::
     for (int k = 0; K > 1 && k < K; ++k) CU(cudaStreamWaitEvent(c->stream, c->join[k], 0));
   const bool both = nspan + nmid > 0 && nrows0 < nb;
   // The row kernel's lists, up before the streams fork: it has to be the first.
+  // (Uploaded before the grids, the span kernel came first at one point in three of
+  // the two-channel sweeps at 1200 and 3000 kept: 10 to 25 ms of 200 to 640 more.)
   int kclusters = 0;
   size_t o_list = 0, o_first = 0;
   if (nrows0 < nb) {
